@@ -11,8 +11,7 @@
 #include <string>
 #include <vector>
 
-#include "hf_device.cuh"
-#include "hf_kernels.cuh"
+#include "hf_cg.cuh"
 
 namespace {
 
@@ -44,6 +43,7 @@ struct DeviceInfo {
     // raises the kernel's dynamic shared-memory limit)
     int res_occ[2][4][2][5];
     int pipe_occ[4][5];   // the single-reduction pressure variant [tiles per group][groups] (-1: not queried yet)
+    bool brick_ready[2][hf::kBrickWideTiles + 1];  // the on-chip pressure solve's kernels whose shared-memory limit is raised
 };
 
 constexpr int kResGroupsMax[4] = {0, 4, 3, 2};   // 256-thread groups per block of the resident variant, by MAXC
@@ -84,6 +84,7 @@ int device_info(DeviceInfo** out) {
         if (!d.coop) return fail(HF_ERR_DEVICE, "device does not support cooperative launches");
         std::memset(d.res_occ, 0xff, sizeof d.res_occ);
         std::memset(d.pipe_occ, 0xff, sizeof d.pipe_occ);
+        std::memset(d.brick_ready, 0, sizeof d.brick_ready);
         d.ready = true;
     }
     *out = &d;
@@ -96,7 +97,8 @@ constexpr size_t kHeadBytes = 256;           // barrier counters, group queue, l
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 struct Layout {
-    size_t head, chunk_begin, tile_begin, maps, partA, partB, mean_part, total;
+    size_t head, chunk_begin, tile_begin, maps, partA, partB, mean_part, streaming;   // streaming: bytes of a plan that only streams
+    size_t brick, arrive, jobs, mail, halo, total;
 };
 
 Layout layout(int S, int C, int T) {
@@ -116,6 +118,17 @@ Layout layout(int S, int C, int T) {
     o = align_up(o + sizeof(double) * 5 * (size_t)T, 256);
     L.mean_part = o;
     o = align_up(o + sizeof(double) * (size_t)C, 256);
+    L.streaming = o;
+    L.brick = o;                     // the on-chip solve: launch, leave and error words
+    o = align_up(o + 256, 256);
+    L.arrive = o;
+    o = align_up(o + sizeof(unsigned) * (size_t)S, 256);
+    L.jobs = o;
+    o = align_up(o + sizeof(int4) * (size_t)S, 256);
+    L.mail = o;                      // a line per unit of a block (one per tile at most), two parities, min(T, kUnits) blocks at most
+    o = align_up(o + 128u * 2u * hf::kBrickWideTiles * (size_t)hf::unit_count(T), 256);
+    L.halo = o;
+    o = align_up(o + sizeof(unsigned long long) * hf::kHaloEntries * (size_t)T, 256);
     L.total = o;
     return L;
 }
@@ -134,6 +147,11 @@ hf::Workspace workspace(const hf_plan* p) {
     w.partA = reinterpret_cast<double*>(b + L.partA);
     w.partB = reinterpret_cast<double*>(b + L.partB);
     w.mean_part = reinterpret_cast<double*>(b + L.mean_part);
+    w.brick = reinterpret_cast<unsigned*>(b + L.brick);
+    w.arrive = reinterpret_cast<unsigned*>(b + L.arrive);
+    w.jobs = reinterpret_cast<int4*>(b + L.jobs);
+    w.mail = reinterpret_cast<ulonglong2*>(b + L.mail);
+    w.halo = reinterpret_cast<unsigned long long*>(b + L.halo);
     w.tiles = p->num_tiles;
     return w;
 }
@@ -215,7 +233,7 @@ int check_plan(const hf_plan* p) {
     if (!p || !p->scenes_host || !p->scenes_dev || !p->work_dev || !p->workspace) return fail(HF_ERR_ARG, "incomplete hf_plan");
     if (p->num_scenes <= 0 || p->num_scenes > hf::kMaxScenes) return fail(HF_ERR_ARG, "num_scenes out of range (1..1024)");
     if (!p->tiles_dev) return fail(HF_ERR_ARG, "incomplete hf_plan (tile table)");
-    if (p->workspace_bytes < layout(p->num_scenes, p->num_chunks, p->num_tiles).total)
+    if (p->workspace_bytes < layout(p->num_scenes, p->num_chunks, p->num_tiles).streaming)
         return fail(HF_ERR_WORKSPACE, "workspace smaller than hf_workspace_bytes()");
     return HF_OK;
 }
@@ -226,6 +244,129 @@ bool any_flag(const hf_plan* p, unsigned f) {
     for (int s = 0; s < p->num_scenes; ++s)
         if ((p->scenes_host[s].flags & HF_FLAG_ACTIVE) && (p->scenes_host[s].flags & f)) return true;
     return false;
+}
+
+// How the on-chip pressure solve shares the blocks among a plan's active scenes: the scenes' jobs in the blocks' common
+// order, the blocks in use, the most tiles that a block owns and the most tiles along k of a scene.
+struct BrickSchedule {
+    std::vector<int4> jobs;   // (scene, first block, blocks, 0)
+    int blocks = 0, tiles = 0, tk = 0;
+};
+
+// the most tiles of a block when `blocks` blocks share a scene of T tiles in whole units (hf_brick.cu)
+int brick_tiles(int T, int blocks) {
+    const int units = hf::unit_count(T);
+    int most = 0;
+    for (int b = 0; b < blocks; ++b)
+        most = std::max(most, hf::unit_first(T, units, (int)((long long)units * (b + 1) / blocks)) -
+                                  hf::unit_first(T, units, (int)((long long)units * b / blocks)));
+    return most;
+}
+
+// False when a scene does not fit: with `cap` kBrickMaxTiles, 148 blocks hold 2220 tiles (an edge of 128 has 2048), with
+// kBrickWideTiles 5328 (an edge of 168 has 5292).
+// Scenes that fit side by side share the blocks in proportion to their tiles.  Otherwise each gets as few blocks as hold
+// it -- the more tiles a block has, the less its reductions weigh -- and the largest come first, each on the contiguous
+// blocks that are free the soonest.
+bool brick_schedule(const hf_plan* p, int sms, int cap, BrickSchedule& out) {
+    const int blocks = std::min(sms, hf::kUnits);
+    out = BrickSchedule();
+    struct Want {
+        int scene, n, T, least, blocks;
+    };
+    std::vector<Want> want;
+    long long total = 0;
+    int least = 0;
+    for (int s = 0; s < p->num_scenes; ++s) {
+        const hf_scene& sc = p->scenes_host[s];
+        if (!(sc.flags & HF_FLAG_ACTIVE)) continue;
+        const int T = tiles_of(sc.n);
+        int nb = (T + cap - 1) / cap;
+        while (nb <= std::min(blocks, T) && brick_tiles(T, nb) > cap) ++nb;
+        if (nb > std::min(blocks, T)) return false;
+        want.push_back(Want{s, sc.n, T, nb, nb});
+        total += T;
+        least += nb;
+        out.tk = std::max(out.tk, (sc.n + hf::kTK - 1) / hf::kTK);
+    }
+    if (want.empty()) return false;
+    if (least <= blocks) {
+        // side by side: the blocks that are left go, one at a time, to the scene whose blocks own the most tiles
+        for (int left = blocks - least; left > 0; --left) {
+            Want* most = nullptr;
+            for (Want& w : want)
+                if (w.blocks < std::min(blocks, w.T) && (!most || (long long)w.T * most->blocks > (long long)most->T * w.blocks)) most = &w;
+            if (!most) break;
+            ++most->blocks;
+        }
+    }
+    std::stable_sort(want.begin(), want.end(), [](const Want& a, const Want& b) { return a.T > b.T; });
+    std::vector<double> until(blocks, 0.0);
+    for (const Want& w : want) {
+        int at = 0;
+        double best = 0.0;
+        for (int f = 0; f + w.blocks <= blocks; ++f) {
+            const double t = *std::max_element(until.begin() + f, until.begin() + f + w.blocks);
+            if (f == 0 || t < best) {
+                best = t;
+                at = f;
+            }
+        }
+        // an iteration takes about 1.6 us of exchanges and 0.35 us a tile; iterations grow like the edge
+        const int most = brick_tiles(w.T, w.blocks);
+        std::fill(until.begin() + at, until.begin() + at + w.blocks, best + w.n * (1.6 + 0.35 * most));
+        out.jobs.push_back(make_int4(w.scene, at, w.blocks, 0));
+        out.blocks = std::max(out.blocks, at + w.blocks);
+        out.tiles = std::max(out.tiles, most);
+    }
+    return true;
+}
+
+bool brick_schedule(const hf_plan* p, int sms, BrickSchedule& out) {
+    return brick_schedule(p, sms, hf::kBrickMaxTiles, out) || brick_schedule(p, sms, hf::kBrickWideTiles, out);
+}
+
+// The on-chip pressure solve of a plan whose scenes all fit.  HF_OK after launching, -1 when it does not apply.
+int launch_brick(const hf_plan* p, DeviceInfo* d, double dt, void* stream) {
+    if (!(p->options & HF_PLAN_MAPS_READY) || p->workspace_bytes < layout(p->num_scenes, p->num_chunks, p->num_tiles).total) return -1;
+    BrickSchedule sched;
+    if (!brick_schedule(p, d->sms, sched)) return -1;
+    for (int s = 0; s < p->num_scenes; ++s) {
+        const hf_scene& sc = p->scenes_host[s];
+        if ((sc.flags & HF_FLAG_ACTIVE) && (!sc.pdiag || !sc.cg_r || !sc.cg_Ap)) return -1;   // scratch of the larger variants
+    }
+    hf::BrickLaunch bl;
+    std::memset(&bl, 0, sizeof bl);
+    bl.jobs = (int)sched.jobs.size();
+    bl.job0 = sched.jobs[0];
+    bl.tiles = sched.tiles;
+    // A block's run of tiles is contiguous in (k, i, j): at most 2 tk of its i faces, all of its j faces and the two k
+    // faces at the run's ends border other blocks.
+    bl.i_pages = (2 * std::min(sched.tk, bl.tiles) + 3) / 4;
+    bl.j_pages = (2 * bl.tiles + 7) / 8;
+    bl.pages = bl.i_pages + bl.j_pages + 1;
+    // as many boxes of face fractions as fit beside the rest and the kernel's own arrays (up to 8 and 18 KB); further
+    // general tiles read the lattices
+    const size_t room = d->smem_optin - (bl.tiles <= hf::kBrickMaxTiles ? 9 : 19) * 1024, base = hf::brick_smem(bl);
+    if (base > room) return -1;
+    bl.boxes = std::min(bl.tiles, (int)((room - base) / hf::brick_box_bytes()));
+    int threads = 0;
+    const void* fn = hf::brick_kernel(bl, &threads);
+    bool& ready = d->brick_ready[bl.boxes < bl.tiles][bl.tiles];
+    if (!ready) {
+        cudaFuncAttributes at;
+        HF_CUDA(cudaFuncGetAttributes(&at, fn), "attributes (on-chip CG)");
+        HF_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(d->smem_optin - at.sharedSizeBytes)),
+                "smem attribute (on-chip CG)");
+        ready = true;
+    }
+    hf::Workspace ws = workspace(p);
+    const hf_scene* scenes = static_cast<const hf_scene*>(p->scenes_dev);
+    const hf::TileItem* tiles = static_cast<const hf::TileItem*>(p->tiles_dev);
+    void* args[] = {(void*)&scenes, (void*)&tiles, (void*)&dt, (void*)&ws, (void*)&bl};
+    HF_CUDA(cudaLaunchCooperativeKernel(fn, dim3(sched.blocks), dim3(threads), args, hf::brick_smem(bl), S(stream)),
+            "cooperative launch (on-chip CG)");
+    return HF_OK;
 }
 
 // The resident variant for a plan with one active scene whose tiles fit one block per SM.  Returns HF_OK after
@@ -247,6 +388,7 @@ int launch_resident(const hf_plan* p, DeviceInfo* d, bool heat, double dt, int s
     // staged and its scratch vectors exist
     const bool pipe = !heat && tma && (p->options & HF_PLAN_SINGLE_REDUCTION_CG) && sc.cg_r && sc.cg_z && sc.cg_Ap &&
                       sc.hdiag && sc.pdiag && sc.cg_p[0] && sc.cg_p[1];
+    if (!heat && !pipe) return -1;
     // tiles per group: the fewest that fit; the single-reduction pressure kernel prefers three (two 256-thread groups
     // of 128 registers per thread: its per-thread state does not fit the 80 registers of a 768-thread block)
     const bool three_first = pipe && !want && tpb > 4;
@@ -299,10 +441,16 @@ int launch_pcg(const hf_plan* p, bool heat, double dt, void* stream) {
             correction = correction || (p->scenes_host[s].flags & HF_FLAG_DEFECT_CORRECTION);
         }
     if (total != p->num_tiles) return fail(HF_ERR_ARG, "plan changed since hf_plan_upload");
-    if (nactive == 1 && !correction && !(p->options & HF_PLAN_STREAMING_CG) &&
-        !(heat && (p->options & HF_PLAN_STREAMING_HEAT))) {
-        rc = launch_resident(p, d, heat, dt, last, stream);
-        if (rc != -1) return rc;
+    if (!correction && !(p->options & HF_PLAN_STREAMING_CG)) {
+        const bool one_reduction = !heat && (p->options & HF_PLAN_SINGLE_REDUCTION_CG);
+        if (nactive == 1 && (heat ? !(p->options & HF_PLAN_STREAMING_HEAT) : one_reduction)) {
+            rc = launch_resident(p, d, heat, dt, last, stream);
+            if (rc != -1) return rc;
+        }
+        if (!heat && nactive > 0) {
+            rc = launch_brick(p, d, dt, stream);
+            if (rc != -1) return rc;
+        }
     }
     static thread_local hf::GroupTable gt;   // 16 KB: kept off the stack; the launch copies it
     gt.count = 0;
@@ -363,6 +511,10 @@ int launch_pcg(const hf_plan* p, bool heat, double dt, void* stream) {
 }  // namespace
 
 namespace hf {
+size_t streaming_workspace_bytes(int num_scenes, int num_chunks, int num_tiles) {
+    return layout(num_scenes, num_chunks, num_tiles).streaming;
+}
+
 int set_error(int code, const char* msg) { return fail(code, msg); }
 
 void plan_offset_tables(const hf_plan* p, int** chunk_begin, int** tile_begin) {
@@ -452,6 +604,14 @@ int hf_plan_upload(hf_plan* p, void* stream) {
     }
     HF_CUDA(cudaMemcpyAsync(b + L.maps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice, S(stream)),
             "upload TMA descriptors");
+    // the on-chip pressure solve's jobs (launch_brick recomputes the same schedule)
+    BrickSchedule sched;
+    DeviceInfo* d = nullptr;
+    int drc = device_info(&d);
+    if (drc) return drc;
+    if (p->num_tiles && brick_schedule(p, d->sms, sched))
+        HF_CUDA(cudaMemcpyAsync(b + L.jobs, sched.jobs.data(), sizeof(int4) * sched.jobs.size(), cudaMemcpyHostToDevice, S(stream)),
+                "upload jobs");
     HF_CUDA(cudaStreamSynchronize(S(stream)), "cudaStreamSynchronize(plan upload)");
     p->options |= HF_PLAN_MAPS_READY;
     return HF_OK;

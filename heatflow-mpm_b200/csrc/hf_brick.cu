@@ -1,0 +1,906 @@
+// hf_brick.cu -- the pressure solve with the CG state on the chip, one scene per team of blocks.
+//
+// Same system, arithmetic and reduction trees as the streaming kernel (hf_cg.cu): mean removal, Jacobi-preconditioned CG
+// warm-started from p, projection, end of the substep (grid.py:235-251, 94-153).  A team of blocks (one 512-thread block
+// per SM) owns a scene's tiles in contiguous runs of whole units; r, A p (and D) of a block's cells live in registers, p
+// and x in shared memory, so an iteration moves only what blocks owe each other.  A plan of several scenes gives every
+// scene a team of its own and a place in the blocks' common order (BrickJobs, hf_api.cu); teams work side by side.
+//
+// What bounds an iteration is latency: two reductions of the whole scene (p.Ap; r.r and r.z) and one halo exchange.  A
+// barrier followed by reading the partials costs a release, an atomic, an acquire poll and another round trip (3450 + 2300
+// cycles for 148 blocks of 512 threads).  Here every value carries its own arrival mark instead, so no fence, counter or
+// barrier is involved and one trip through L2 does:
+//   * reductions: a block adds its tiles' partials into unit sums and posts each on a 128-byte line of its own as {low
+//     word, tag, high word, tag}, self-validating 8-byte halves; every member polls all lines of its team.  A line that
+//     is being polled takes one store, of one warp instruction: measured alone, 148 blocks and two values, 1830 to 2400
+//     cycles; two stores to the line 2200 to 4300, lines that several blocks write 10,000 and more.
+//   * halo: z of the cells on faces that a tile shares with another block's tile, as {z, tag} words that the neighbour
+//     polls (again one store for each run of 32).  Each block advances its own copy of p there by the owner's operations
+//     on the owner's values.
+// Tags name launch, job and step, so nothing has to be cleared between launches.  A line alternates with the parity of
+// the step: a member posts step s + 2 only after step s + 1, which every member posted after reading step s.
+#include "hf_cg.cuh"
+
+namespace hf {
+
+constexpr int kFaceBox = 5 * 256 + 4 * 9 * 32 + 4 * 8 * 33;   // floats of one tile's face fractions
+constexpr int kBoxY = 5 * 256, kBoxZ = kBoxY + 4 * 9 * 32;
+constexpr int kHaloRows = 2 * 8 + 2 * 4 + 2;                  // 32-value rows of a tile's six faces
+constexpr int kPollWarps = (kUnits + 31) / 32;                // warps that wait for the other blocks' sums
+                                                              // (the others fetch the halo)
+
+// first entry of face f (i-, i+, j-, j+, k-, k+) in a tile's halo slot
+__device__ __forceinline__ int face_entry(int f) { return f < 2 ? f * 256 : f < 4 ? 512 + (f - 2) * 128 : 768 + (f - 4) * 32; }
+
+// One tile of the block: nb[f] is the shared-memory offset of the values beyond face f, in the core of another tile of
+// the block, in a halo page, or (domain face) the tile's own cells.  Offsets are laid out so that every neighbour of
+// cell m lies at nb + m * 256 + (j * 32 | lane), whatever it points to.
+struct BrickTile {
+    int i0, j0, k0;
+    int nb[6];
+    int remote;   // bit f: face f borders a tile of another block
+    int face;     // offset of the tile's face fractions, or -1: read from the lattices
+    int unit;     // all cells in the domain and every fraction between them 1
+    int slot;     // first entry of the tile's halo slot
+};
+
+__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_halves(ulonglong2* p, double v, unsigned tag) {
+    const unsigned long long t = (unsigned long long)tag << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(t | (unsigned)__double2loint(v)),
+                 "l"(t | (unsigned)__double2hiint(v))
+                 : "memory");
+}
+__device__ __forceinline__ ulonglong2 ld_halves(const ulonglong2* p) {
+    ulonglong2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+    return v;
+}
+
+// A bounded wait's clock: false once the limit has passed or another block has given up (which sets err).
+struct Patience {
+    unsigned long long t0 = 0;
+    unsigned spins = 0;
+    __device__ __forceinline__ bool more(int* err) {
+        if (++spins & 63u) return true;
+        if (*(volatile int*)err) return false;
+        const unsigned long long now = global_timer_ns();
+        if (!t0) t0 = now;
+        if (now - t0 <= c_wait_limit_ns) return true;
+        atomicExch(err, 1);
+        return false;
+    }
+};
+
+// The warp sums of K values per lane, value by value the butterfly of offsets 16, 8, 4, 2, 1: while more than one value is
+// left, the lanes of a pair share them (each keeps half and adds the other's), which adds the same numbers in the same
+// order as K separate butterflies, with half the exchanges or fewer.  Returns the value's index; its sum is in v[0].
+template <int K, int P, int OFF>
+__device__ __forceinline__ void fold(double* v, int lane, int& index) {
+    if constexpr (OFF > 0) {
+        if constexpr (P == 1) {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], OFF);
+            fold<1, 1, OFF / 2>(v, lane, index);
+        } else {
+            constexpr int H = P / 2;
+            const bool hi = lane & OFF;
+#pragma unroll
+            for (int i = 0; i < H; ++i) {
+                if (i >= K) continue;
+                const double a = v[i], b = i + H < K ? v[i + H] : 0.0;
+                v[i] = (hi ? b : a) + __shfl_xor_sync(0xffffffffu, hi ? a : b, OFF);
+            }
+            index += hi ? H : 0;
+            fold<(K < H ? K : H), H, OFF / 2>(v, lane, index);
+        }
+    }
+}
+__host__ __device__ constexpr int pow2_above(int k) { return k <= 1 ? 1 : 2 * pow2_above((k + 1) / 2); }
+
+// a / b rounded to double: Newton's iteration for 1 / b from its binary32 value, then the quotient with Markstein's
+// correction (IBM J. Res. Dev. 34(1), 1990; the remainder a - q b is exact with one FMA).  150 cycles from operands to
+// result instead of 410 to 700 for the operator, and the scalars of an iteration wait for two of them.  Operands outside
+// [2^-100, 2^100] take the operator.
+__device__ __forceinline__ double quotient(double a, double b) {
+    const double ab = fabs(b), aa = fabs(a);
+    if (!(ab >= 0x1p-100 && ab <= 0x1p100 && aa >= 0x1p-100 && aa <= 0x1p100)) return a / b;
+    double y = (double)__frcp_rn((float)b);
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    const double q = a * y;
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+
+// div_rn of four values at once: one test of their range instead of four.  Zeros (every cell outside the domain has one)
+// stay on the short way: their quotient comes out as zero there too.
+__device__ __forceinline__ void div_rn4(float (&x)[4], const DivBy& d) {
+    float low[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) low[m] = x[m] == 0.0f ? 1.0f : fabsf(x[m]);
+    const float lo = fminf(fminf(low[0], low[1]), fminf(low[2], low[3]));
+    const float hi = fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3])));
+    if (lo >= 0x1p-96f && hi <= 0x1p96f) {   // a NaN among them passes through both ways
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const float q = __fmaf_rn(x[m], d.zh, __fmul_rn(x[m], d.zl));
+            x[m] = __fmaf_rn(__fmaf_rn(-q, d.y, x[m]), d.zh, q);
+        }
+    } else {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) x[m] = div_rn(x[m], d);
+    }
+}
+
+// A block's place in a team.  A block owns at most as many units as tiles.
+constexpr int kLines = kBrickWideTiles;        // lines of a block and parity
+struct Team {
+    int units, mine;                           // units of the scene and of this block,
+    const int* begin;                          // the first tile of each of these (and the end)
+    ulonglong2* post;                          // this block's lines (two parities)
+    const ulonglong2* poll;                    // the line of unit threadIdx.x
+    unsigned base;                             // launch and job part of the tags
+    int* err;
+};
+
+// The scene sums of K components from the tile partials in red[(c * 8 + warp) * NT + tile], handed to `derive` in the first
+// thread, which leaves what the block needs in shared memory (every thread deriving it for itself made 96^3 5 % slower).
+// `before` is what the warps that do not wait for the sums do meanwhile.  False, in every thread, when a wait of any
+// thread gave up (bad).
+template <int K, int NT, class Before, class Derive>
+__device__ __forceinline__ bool exchange(const Team& team, int nt, unsigned& step, const double* red, double* tsum,
+                                         double (*sums)[8], int& bad, Before before, Derive derive) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    ++step;
+    const unsigned tag = team.base | (step & 0x3ffu);
+    __syncthreads();
+    if (warp == 0 && !(step == 1 && (int)blockIdx.x == c_absent_block)) {
+        // tile partials (8 warps in order), then the unit sums (tiles in order): lane 4 u + c has component c of unit u,
+        // so a unit's line is written by one instruction
+        // (absent tiles as +0.0, which changes nothing).  All loads come before the additions.
+        for (int tile = lane; tile < nt; tile += 32) {
+            double w[K][8];
+#pragma unroll
+            for (int c = 0; c < K; ++c)
+#pragma unroll
+                for (int q = 0; q < 8; ++q) w[c][q] = red[(c * 8 + q) * NT + tile];
+#pragma unroll
+            for (int c = 0; c < K; ++c) {
+                double s = 0.0;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) s += w[c][q];
+                tsum[c * NT + tile] = s;
+            }
+        }
+        __syncwarp();
+        for (int u = lane >> 2; u < team.mine; u += 8) {
+            const int c = lane & 3, a = team.begin[u], e = team.begin[u + 1];
+            if (c >= K) continue;
+            constexpr int kAtOnce = NT <= 15 ? NT : 12;
+            double s = 0.0;
+            for (int q0 = a; q0 < e; q0 += kAtOnce) {
+                double v[kAtOnce];
+#pragma unroll
+                for (int q = 0; q < kAtOnce; ++q) v[q] = q0 + q < e ? tsum[c * NT + q0 + q] : 0.0;
+#pragma unroll
+                for (int q = 0; q < kAtOnce; ++q) s += v[q];
+            }
+            st_halves(team.post + ((step & 1u) * kLines + u) * 8 + c, s, tag);
+        }
+    }
+    if (warp >= kPollWarps) {
+        before();
+    } else {
+        double v[K];
+#pragma unroll
+        for (int c = 0; c < K; ++c) v[c] = 0.0;
+        // The warp leaves the loop together, by vote: lanes that left it one by one would stay apart until the next barrier
+        // and issue every following shuffle group by group (250 cycles each instead of 33).
+        const ulonglong2* line = team.poll + (step & 1u) * kLines * 8;
+        bool here = t >= team.units;
+        Patience patience;
+        for (;;) {
+            if (!here) {
+                ulonglong2 q[K];
+#pragma unroll
+                for (int c = 0; c < K; ++c) q[c] = ld_halves(line + c);
+                here = true;
+#pragma unroll
+                for (int c = 0; c < K; ++c) {
+                    here = here && (unsigned)(q[c].x >> 32) == tag && (unsigned)(q[c].y >> 32) == tag;
+                    v[c] = __hiloint2double((int)(unsigned)q[c].y, (int)(unsigned)q[c].x);
+                }
+            }
+            if (__all_sync(0xffffffffu, here)) break;
+            if (__any_sync(0xffffffffu, !patience.more(team.err))) {
+                bad = 1;
+                break;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < K; ++c) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
+            if (lane == 0) sums[c][warp] = v[c];
+        }
+        asm volatile("bar.sync 15, %0;" ::"n"(kPollWarps * 32) : "memory");
+        if (t == 0) {
+            double tot[K];
+#pragma unroll
+            for (int c = 0; c < K; ++c) {
+                double s = 0.0;
+#pragma unroll
+                for (int w = 0; w < kPollWarps; ++w) s += sums[c][w];
+                tot[c] = s;
+            }
+            derive(tot);
+        }
+    }
+    return !__syncthreads_or(bad);
+}
+
+// G groups of 256 threads with up to Q tiles each.  With one tile a thread keeps all of its cells' state in registers (p also
+// in shared memory, for the neighbours); up to three it keeps D; beyond, D of a unit tile follows from the number of a
+// cell's faces, and other tiles read it back.
+// Q = 0, for large scenes: only p stays on the chip.  r, A p and x are read and written where they are used, by the thread
+// that owns the cell (28 bytes of L2 traffic per cell and iteration; the streaming kernel moves 60 and p's halo from HBM).
+template <int G, int Q>
+__global__ void __launch_bounds__(256 * G, 1)
+    k_brick(const hf_scene* __restrict__ scenes, const TileItem* __restrict__ tiles, double dt_d, Workspace ws, BrickLaunch bl) {
+    constexpr bool kWide = Q == 0;
+    constexpr int QR = kWide ? 1 : Q;                         // tiles a thread holds at a time
+    constexpr int NT = kWide ? kBrickWideTiles : G * Q;
+    constexpr int kWarps = 8 * G, kRowWarps = kWarps - kPollWarps;
+    constexpr int kRowsEach = kWide ? 16 : G == 4 ? 3 : Q <= 2 ? 6 : 10;   // halo rows that a warp keeps while the sums are on their way
+    constexpr bool kKeepD = !kWide && Q <= 3, kKeepX = NT <= 2;
+    constexpr bool kLattice = kWide || NT > 9;                // general tiles may find no box for their fractions
+    extern __shared__ __align__(16) float sm[];   // p, x (1024 floats a tile each), halo pages, face boxes
+    __shared__ BrickTile tt[NT];
+    __shared__ int2 rows[NT * kHaloRows];         // (entry in the neighbour's slot, shared offset; bit 30: a k face)
+    __shared__ double red[3 * NT * 8];
+    __shared__ double tsum[3 * NT];
+    __shared__ int ubegin[kLines + 1];
+    __shared__ float kface[2 * 32];               // values of the run's two k faces on their way out
+    __shared__ double sums[3][8];
+    __shared__ LocalScene Ls;
+    __shared__ float dtab[8];
+    __shared__ int s_count[5];                    // i planes, j slots, k columns, rows, face boxes in use
+    const int g = threadIdx.x >> 8, lt = threadIdx.x & 255, lane = lt & 31, row = lt >> 5, warp = threadIdx.x >> 5;
+    int* const err = reinterpret_cast<int*>(ws.brick + 2);
+    const unsigned launch = *(volatile unsigned*)ws.brick;
+    const int X = kWide ? 0 : bl.tiles * 1024;    // x follows p (wide: takes p's place at the end)
+    const int pages = bl.tiles * (kWide ? 1024 : 2048), boxes = pages + bl.pages * 1024;
+    int bad = 0;                                  // a wait of this thread gave up
+    int left = -1, left_nb = 0;                   // the job before and its blocks
+
+    for (int job = 0; job < bl.jobs; ++job) {
+        const int4 J = bl.jobs == 1 ? bl.job0 : ws.jobs[job];   // scene, first block, blocks
+        if ((int)blockIdx.x < J.y || (int)blockIdx.x >= J.y + J.z) continue;
+        const hf_scene& S = scenes[J.x];
+        const bool leader = (int)blockIdx.x == J.y;
+        if (__syncthreads_or(*(volatile int*)err)) {   // a wait gave up earlier in this launch: the scene stays unsolved
+            if (leader && threadIdx.x == 0) S.state->status |= HF_SCENE_BARRIER_TIMEOUT;
+            continue;
+        }
+        Team team;
+        const int b = (int)blockIdx.x - J.y, tb = ws.tile_begin[J.x];
+        const int T = ws.tile_begin[J.x + 1] - tb;
+        team.units = unit_count(T);
+        const int u0 = unit_first(team.units, J.z, b), u1 = unit_first(team.units, J.z, b + 1);
+        const int c0 = unit_first(T, team.units, u0), c1 = unit_first(T, team.units, u1), nt = c1 - c0;
+        team.mine = u1 - u0;
+        team.begin = ubegin;
+        team.post = ws.mail + (size_t)blockIdx.x * 2 * kLines * 8;
+        {
+            // the owner of unit t and the unit's place among its units
+            const int t = (int)threadIdx.x < team.units ? threadIdx.x : 0, o = (int)(((long long)(t + 1) * J.z - 1) / team.units);
+            team.poll = ws.mail + ((size_t)(J.y + o) * 2 * kLines + t - unit_first(team.units, J.z, o)) * 8;
+        }
+        team.base = launch << 20 | (unsigned)job << 10;
+        team.err = err;
+        unsigned step = 0, pub = 0;
+        bool ok = true;
+        const int n = S.n, par = S.state->parity;
+        const float h = (float)S.h, hh = __fmul_rn(h, h);
+        const DivBy hhd = div_by(hh);
+        const int ti = (n + kTI - 1) / kTI, tj = (n + kTJ - 1) / kTJ, tk = (n + kTK - 1) / kTK;
+
+        // ------------------------------------------------------------------------------------ the block's tiles
+        if (threadIdx.x < 5) s_count[threadIdx.x] = 0;
+        if ((int)threadIdx.x <= team.mine) ubegin[threadIdx.x] = unit_first(T, team.units, u0 + threadIdx.x) - c0;
+        if (threadIdx.x < 7) dtab[threadIdx.x] = __fdiv_rn(hh, maxf_((float)threadIdx.x, 1.0e-12f));
+        __syncthreads();
+        if (threadIdx.x < nt) {
+            const int q = threadIdx.x, c = c0 + q;
+            const TileItem it = tiles[tb + c];
+            BrickTile t;
+            t.i0 = it.i0;
+            t.j0 = it.j0;
+            t.k0 = it.k0;
+            t.slot = (tb + c) * kHaloEntries;
+            t.remote = 0;
+            t.face = -1;
+            t.unit = it.i0 + kTI <= n && it.j0 + kTJ <= n && it.k0 + kTK <= n;
+            const bool there[6] = {it.i0 > 0, it.i0 / kTI + 1 < ti, it.j0 > 0, it.j0 / kTJ + 1 < tj, it.k0 > 0, it.k0 / kTK + 1 < tk};
+            const int away[6] = {-tk, tk, -tk * ti, tk * ti, -1, 1};
+            // offsets within the neighbour's core, and within the tile's own (domain faces: the cell itself)
+            const int far[6] = {768, 0, 224, 0, 31, 0}, own[6] = {0, 768, 0, 224, 0, 31};
+#pragma unroll
+            for (int f = 0; f < 6; ++f) {
+                const int o = c + away[f];
+                if (!there[f]) {
+                    t.nb[f] = q * 1024 + own[f];
+                } else if (o >= c0 && o < c1) {
+                    t.nb[f] = (o - c0) * 1024 + far[f];
+                } else {
+                    t.remote |= 1 << f;
+                    const int kind = f >> 1, at = atomicAdd(&s_count[kind], 1);
+                    // a page holds 4 planes (i faces), 8 slots of a row per m (j faces) or 32 columns (k faces)
+                    const int room = kind == 0 ? 4 * bl.i_pages : kind == 1 ? 8 * bl.j_pages : 32 * (bl.pages - bl.i_pages - bl.j_pages);
+                    if (at >= room) {
+                        atomicExch(err, 1);   // cannot happen: the launch sizes the pages for its longest run
+                        t.nb[f] = q * 1024 + own[f];
+                        continue;
+                    }
+                    const int page = pages + (kind == 0 ? at / 4 : kind == 1 ? bl.i_pages + at / 8 : bl.i_pages + bl.j_pages + at / 32) * 1024;
+                    t.nb[f] = page + (kind == 0 ? (at % 4) * 256 : kind == 1 ? (at % 8) * 32 : at % 32);
+                    const int src = (tb + o) * kHaloEntries + face_entry(f ^ 1), count = kind == 0 ? 8 : kind == 1 ? 4 : 1;
+                    const int r0 = atomicAdd(&s_count[3], count);
+                    for (int r = 0; r < count; ++r)
+                        rows[r0 + r] = make_int2(src + r * 32, kind == 0 ? t.nb[f] + r * 32 : kind == 1 ? t.nb[f] + r * 256
+                                                                                                         : t.nb[f] | 1 << 30);
+                }
+            }
+            tt[q] = t;
+        }
+        if (left >= 0 && threadIdx.x == 0) {
+            // everyone has read this block's last sums of the job before: its lines may be written again
+            Patience patience;
+            while (ld_acquire_u32(ws.arrive + left) < (unsigned)left_nb)
+                if (!patience.more(err)) {
+                    bad = 1;
+                    break;
+                }
+        }
+        // the pressure rhs mean (grid.py:238-241) from the divergence stage's chunk sums: 256 threads in strides, warp
+        // butterfly, 8 warps in order
+        float mean;
+        {
+            double m = 0.0;
+            if (threadIdx.x < kThreads)
+                for (int c = ws.chunk_begin[J.x] + threadIdx.x; c < ws.chunk_begin[J.x + 1]; c += kThreads) m += ws.mean_part[c];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+            __syncthreads();
+            if (lane == 0 && warp < 8) sums[0][warp] = m;
+            __syncthreads();
+            m = 0.0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) m += sums[0][q];
+            mean = __double2float_rn(m / ((double)n * n * n));
+        }
+        const int nrows = s_count[3];
+        auto post = [&](const BrickTile& T, const float (&v)[4], unsigned tag) {
+            const int rem = T.remote;
+            if (!rem) return;
+            unsigned long long* to = ws.halo + T.slot;
+            const unsigned long long mark = (unsigned long long)tag << 32;
+            auto put = [&](int e, float x) { st_relaxed(to + e, mark | __float_as_uint(x)); };
+            if (rem & 1) put(lt, v[0]);
+            if (rem & 2) put(256 + lt, v[3]);
+            if ((rem & 4) && row == 0)
+#pragma unroll
+                for (int m = 0; m < 4; ++m) put(512 + m * 32 + lane, v[m]);
+            if ((rem & 8) && row == 7)
+#pragma unroll
+                for (int m = 0; m < 4; ++m) put(640 + m * 32 + lane, v[m]);
+            // a k face (the run's first or last) comes from eight warps: gathered here, sent by one (post_k, after a barrier)
+            if ((rem & 16) && lane == 0)
+#pragma unroll
+                for (int m = 0; m < 4; ++m) kface[m * 8 + row] = v[m];
+            if ((rem & 32) && lane == 31)
+#pragma unroll
+                for (int m = 0; m < 4; ++m) kface[32 + m * 8 + row] = v[m];
+        };
+        auto post_k = [&](unsigned tag) {
+            const int e = warp - kPollWarps;
+            if (e > 1) return;
+            const BrickTile& T = tt[e ? nt - 1 : 0];
+            if (T.remote & (16 << e))
+                st_relaxed(ws.halo + T.slot + 768 + e * 32 + lane, (unsigned long long)tag << 32 | __float_as_uint(kface[e * 32 + lane]));
+        };
+        // The halo's rows.  fetch: the warps that do not wait for the sums wait for theirs, up to kRowsEach rows each, into
+        // registers.  take: every value goes to its place through apply(place, value).
+        float ahead[kRowsEach];
+        auto await = [&](int r, unsigned tag, unsigned long long v) {
+            const unsigned long long* from = ws.halo + rows[r].x + lane;
+            Patience patience;
+            while (__any_sync(0xffffffffu, (unsigned)(v >> 32) != tag)) {   // the warp stays together
+                if (__any_sync(0xffffffffu, !patience.more(err))) {
+                    bad = 1;
+                    break;
+                }
+                v = ld_relaxed(from);
+            }
+            return __uint_as_float((unsigned)v);
+        };
+        auto fetch = [&](unsigned tag) {
+            post_k(tag);
+            unsigned long long v[kRowsEach];
+#pragma unroll
+            for (int u = 0; u < kRowsEach; ++u) {
+                const int r = warp - kPollWarps + u * kRowWarps;
+                v[u] = r < nrows ? ld_relaxed(ws.halo + rows[r].x + lane) : 0ull;
+            }
+#pragma unroll
+            for (int u = 0; u < kRowsEach; ++u) {
+                const int r = warp - kPollWarps + u * kRowWarps;
+                if (r < nrows) ahead[u] = await(r, tag, v[u]);
+            }
+        };
+        auto take = [&](unsigned tag, auto apply) {
+            auto place = [&](int r) {
+                const int at = rows[r].y;
+                return (at >> 30) & 1 ? (at & 0x3fffffff) + (lane >> 3) * 256 + (lane & 7) * 32 : at + lane;
+            };
+            if (warp >= kPollWarps) {
+#pragma unroll
+                for (int u = 0; u < kRowsEach; ++u) {
+                    const int r = warp - kPollWarps + u * kRowWarps;
+                    if (r < nrows) apply(sm[place(r)], ahead[u]);
+                }
+            }
+            for (int r = kRowWarps * kRowsEach + warp; r < nrows; r += kWarps)
+                apply(sm[place(r)], await(r, tag, ld_relaxed(ws.halo + rows[r].x + lane)));
+        };
+
+        // the warp's sums of K components of its tiles (one: q, wide; else the group's) go to red
+        auto stash = [&](int q, auto& part) {
+            constexpr int N = (int)(sizeof(part) / sizeof(double)), P = pow2_above(N);
+            static_assert(P <= 32, "one value per lane at most");
+            int index = 0;
+            fold<N, P, 16>(part, lane, index);
+            const int at = kWide ? q : G * (index % QR) + g;
+            if (index < N && (lane & (32 / P - 1)) == 0 && at < nt) red[(index / QR * 8 + row) * NT + at] = part[0];
+        };
+        // ------------------------------------------------------------------------------------ set-up
+        float r[4 * QR], ap[4 * QR], dg[kKeepD ? 4 * QR : 1], xr[kKeepX ? 4 * QR : 1], pr[kKeepX ? 4 * QR : 1];
+        const int turns = kWide ? (nt - g + G - 1) / G : Q;   // of the loops over a group's tiles; unrolled unless wide
+        {
+            // x0 = p, b = rhs - mean, D (k_jacobi), r0 = b - A x0, z0 = D r0; a tile with a fraction other than 1 is general
+            double part[3 * QR];
+#pragma unroll QR
+            for (int turn = 0; turn < turns; ++turn) {
+                const int s = kWide ? 0 : turn, q = G * turn + g;
+                part[s] = part[QR + s] = part[2 * QR + s] = 0.0;
+                float z4[4];
+                if (q < nt) {
+                    const TileItem it{0, tt[q].i0, tt[q].j0, tt[q].k0};
+                    bool one = true;
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        const int e = s * 4 + m;
+                        const Cell cl = tile_cell(it, n, lt, m);
+                        float xc = 0.0f, z = 0.0f;
+                        r[e] = ap[e] = 0.0f;
+                        if (kKeepD) dg[e] = 0.0f;
+                        if (cl.ok) {
+                            const int t = cl.t, nn = n * n;
+                            const bool in[6] = {cl.i > 0, cl.i < n - 1, cl.j > 0, cl.j < n - 1, cl.k > 0, cl.k < n - 1};
+                            const int away[6] = {-nn, nn, -n, n, -1, 1};
+                            const float* at[6] = {S.ax + uidx_(n, cl.i, cl.j, cl.k), S.ax + uidx_(n, cl.i + 1, cl.j, cl.k),
+                                                  S.ay + vidx_(n, cl.i, cl.j, cl.k), S.ay + vidx_(n, cl.i, cl.j + 1, cl.k),
+                                                  S.az + widx_(n, cl.i, cl.j, cl.k), S.az + widx_(n, cl.i, cl.j, cl.k + 1)};
+                            float af[6], xn[6];
+                            xc = S.p[t];
+#pragma unroll
+                            for (int f = 0; f < 6; ++f) {
+                                af[f] = __ldg(at[f]);
+                                xn[f] = S.p[in[f] ? t + away[f] : t];
+                            }
+                            float bv = S.rhs[t];
+                            if (mean != 0.0f) {
+                                bv = __fsub_rn(bv, mean);
+                                S.rhs[t] = bv;
+                            }
+                            float sa = 0.0f, acc = 0.0f;
+#pragma unroll
+                            for (int f = 0; f < 6; ++f)
+                                if (in[f]) {
+                                    sa = __fadd_rn(sa, af[f]);
+                                    acc = __fadd_rn(acc, __fmul_rn(af[f], __fsub_rn(xc, xn[f])));
+                                    one = one && af[f] == 1.0f;
+                                }
+                            const float d = __fdiv_rn(hh, maxf_(sa, 1.0e-12f)), rv = __fsub_rn(bv, __fdiv_rn(acc, hh));
+                            z = __fmul_rn(d, rv);
+                            r[e] = rv;
+                            if (kWide) S.cg_r[t] = rv;
+                            if (kKeepD) dg[e] = d;
+                            else S.pdiag[t] = d;
+                            part[s] += (double)bv * (double)bv;
+                            part[QR + s] += (double)rv * (double)rv;
+                            part[2 * QR + s] += (double)rv * (double)z;
+                        }
+                        z4[m] = z;
+                        if (kKeepX) {
+                            xr[e] = xc;
+                            pr[e] = z;
+                        } else if (!kWide) {
+                            sm[X + q * 1024 + m * 256 + lt] = xc;
+                        }
+                        sm[q * 1024 + m * 256 + lt] = z;
+                    }
+                    if (!one) tt[q].unit = 0;
+                    post(tt[q], z4, team.base | (pub + 1));
+                } else {
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        r[s * 4 + m] = ap[s * 4 + m] = 0.0f;
+                        if (kKeepD) dg[s * 4 + m] = 0.0f;
+                        if (kKeepX) xr[s * 4 + m] = pr[s * 4 + m] = 0.0f;
+                    }
+                }
+                if (kWide) stash(q, part);
+            }
+            ++pub;
+            if (!kWide) stash(g, part);
+        }
+        {
+            ok = exchange<3, NT>(team, nt, step, red, tsum, sums, bad, [&] { fetch(team.base | pub); },
+                                 [&](const double (&tot)[3]) {
+                                     init_scalars(Ls, S, false, tot, n * n * n);
+                                     Ls.mean = (double)mean;
+                                 });
+        }
+        // face fractions of the general tiles, zero where a face has no cell on one side (those terms drop out)
+        for (int q = g; q < nt; q += G) {
+            if (tt[q].unit) continue;   // uniform in the group
+            if (lt == 0) {
+                const int at = atomicAdd(&s_count[4], 1);
+                tt[q].face = at < bl.boxes ? boxes + at * kFaceBox : -1;
+            }
+            asm volatile("bar.sync %0, 256;" ::"r"(g + 1) : "memory");
+            const int to = tt[q].face, i0 = tt[q].i0, j0 = tt[q].j0, k0 = tt[q].k0;
+            if (to < 0) continue;
+            for (int e = lt; e < kFaceBox; e += 256) {
+                float v = 0.0f;
+                if (e < kBoxY) {
+                    const int i = i0 + (e >> 8), j = j0 + ((e >> 5) & 7), k = k0 + (e & 31);
+                    if (i > 0 && i < n && j < n && k < n) v = __ldg(S.ax + uidx_(n, i, j, k));
+                } else if (e < kBoxZ) {
+                    const int w = e - kBoxY, i = i0 + w / 288, j = j0 + (w % 288) / 32, k = k0 + (w & 31);
+                    if (j > 0 && i < n && j < n && k < n) v = __ldg(S.ay + vidx_(n, i, j, k));
+                } else {
+                    const int w = e - kBoxZ, i = i0 + w / 264, j = j0 + (w % 264) / 33, k = k0 + w % 33;
+                    if (k > 0 && i < n && j < n && k < n) v = __ldg(S.az + widx_(n, i, j, k));
+                }
+                sm[to + e] = v;
+            }
+        }
+        __syncthreads();
+        // the first of a tile's four cells, and which of them the domain has
+        auto first_cell = [&](const BrickTile& T, int& cells) {
+            const int j = T.j0 + row, k = T.k0 + lane;
+            cells = j < n && k < n ? min(4, n - T.i0) : 0;
+            return (T.i0 * n + j) * n + k;
+        };
+        bool live = ok && Ls.live;
+        int kit = 0;
+        float beta = 0.0f;
+
+        // D of the four cells of a tile when it is not kept (a unit tile's from the number of faces in the domain)
+        auto diag = [&](const BrickTile& T, int s, float (&d)[4]) {
+            if constexpr (kKeepD) {
+#pragma unroll
+                for (int m = 0; m < 4; ++m) d[m] = dg[s * 4 + m];
+            } else {
+                const int j = T.j0 + row, k = T.k0 + lane;
+                if (T.unit) {
+                    const int c = 6 - (j == 0) - (j == n - 1) - (k == 0) - (k == n - 1);
+                    d[1] = d[2] = dtab[c];
+                    d[0] = dtab[c - (T.i0 == 0)];
+                    d[3] = dtab[c - (T.i0 + 4 == n)];
+                } else {
+                    const bool in = j < n && k < n;
+                    const float* from = S.pdiag + (T.i0 * n + j) * n + k;
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) d[m] = in && T.i0 + m < n ? from[m * n * n] : 0.0f;
+                }
+            }
+        };
+
+        // ------------------------------------------------------------------------------------ iterations
+        while (live) {
+            ++kit;
+            // p = z + beta p: the halo's copies and the block's own cells (the first p is z, placed by the set-up)
+            take(team.base | (pub & 0x3ffu), [&](float& pb, float z) { pb = kit == 1 ? z : __fadd_rn(z, __fmul_rn(beta, pb)); });
+            if (kit > 1) {
+#pragma unroll (kWide ? 3 : QR)
+                for (int turn = 0; turn < turns; ++turn) {
+                    const int s = kWide ? 0 : turn, q = G * turn + g;
+                    if (q >= nt) continue;
+                    float d[4], rv[4];
+                    diag(tt[q], s, d);
+                    float* core = sm + q * 1024 + lt;
+                    int cells;
+                    const int t = first_cell(tt[q], cells);
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) rv[m] = !kWide ? r[s * 4 + m] : m < cells ? S.cg_r[t + m * n * n] : 0.0f;
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        const float pv = __fadd_rn(__fmul_rn(d[m], rv[m]), __fmul_rn(beta, kKeepX ? pr[s * 4 + m] : core[m * 256]));
+                        core[m * 256] = pv;
+                        if (kKeepX) pr[s * 4 + m] = pv;
+                    }
+                }
+            }
+            __syncthreads();
+            double pAp[QR];
+#pragma unroll QR
+            for (int turn = 0; turn < turns; ++turn) {
+                const int s = kWide ? 0 : turn, q = G * turn + g;
+                pAp[s] = 0.0;
+                if (q >= nt) continue;
+                const BrickTile& T = tt[q];
+                const int core = q * 1024 + lt;
+                const float* lo_j = sm + (row == 0 ? T.nb[2] + lane : core - 32);
+                const float* hi_j = sm + (row == 7 ? T.nb[3] + lane : core + 32);
+                const float* lo_k = sm + (lane == 0 ? T.nb[4] + row * 32 : core - 1);
+                const float* hi_k = sm + (lane == 31 ? T.nb[5] + row * 32 : core + 1);
+                float p[6];   // the column i0 - 1 .. i0 + 4
+                p[0] = sm[T.nb[0] + lt];
+                p[5] = sm[T.nb[1] + lt];
+#pragma unroll
+                for (int m = 0; m < 4; ++m) p[m + 1] = kKeepX ? pr[s * 4 + m] : sm[core + m * 256];
+                float a[4];
+                if (T.unit) {
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        const float pc = p[m + 1];
+                        float acc = __fadd_rn(__fsub_rn(pc, p[m]), __fsub_rn(pc, p[m + 2]));
+                        acc = __fadd_rn(acc, __fsub_rn(pc, lo_j[m * 256]));
+                        acc = __fadd_rn(acc, __fsub_rn(pc, hi_j[m * 256]));
+                        acc = __fadd_rn(acc, __fsub_rn(pc, lo_k[m * 256]));
+                        a[m] = __fadd_rn(acc, __fsub_rn(pc, hi_k[m * 256]));
+                    }
+                } else if (!kLattice || T.face >= 0) {
+                    const float* fx = sm + T.face + lt;
+                    const float* fy = sm + T.face + kBoxY + lt;
+                    const float* fz = sm + T.face + kBoxZ + row * 33 + lane;
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        const float pc = p[m + 1];
+                        float acc = __fmul_rn(fx[m * 256], __fsub_rn(pc, p[m]));
+                        acc = __fadd_rn(acc, __fmul_rn(fx[m * 256 + 256], __fsub_rn(pc, p[m + 2])));
+                        acc = __fadd_rn(acc, __fmul_rn(fy[m * 288], __fsub_rn(pc, lo_j[m * 256])));
+                        acc = __fadd_rn(acc, __fmul_rn(fy[m * 288 + 32], __fsub_rn(pc, hi_j[m * 256])));
+                        acc = __fadd_rn(acc, __fmul_rn(fz[m * 264], __fsub_rn(pc, lo_k[m * 256])));
+                        a[m] = __fadd_rn(acc, __fmul_rn(fz[m * 264 + 1], __fsub_rn(pc, hi_k[m * 256])));
+                    }
+                } else {
+                    // no box left: the fractions from the lattices, all requested before the first is used
+                    const int i0 = T.i0, j = T.j0 + row, k = T.k0 + lane;
+                    const bool in = j < n && k < n;
+                    float fx[5], fy[8], fz[8];
+#pragma unroll
+                    for (int m = 0; m < 5; ++m)
+                        fx[m] = in && i0 + m > 0 && i0 + m < n ? __ldg(S.ax + uidx_(n, i0 + m, j, k)) : 0.0f;
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        const bool im = in && i0 + m < n;
+                        fy[m] = im && j > 0 ? __ldg(S.ay + vidx_(n, i0 + m, j, k)) : 0.0f;
+                        fy[4 + m] = im && j < n - 1 ? __ldg(S.ay + vidx_(n, i0 + m, j + 1, k)) : 0.0f;
+                        fz[m] = im && k > 0 ? __ldg(S.az + widx_(n, i0 + m, j, k)) : 0.0f;
+                        fz[4 + m] = im && k < n - 1 ? __ldg(S.az + widx_(n, i0 + m, j, k + 1)) : 0.0f;
+                    }
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        const float pc = p[m + 1];
+                        float acc = __fmul_rn(fx[m], __fsub_rn(pc, p[m]));
+                        acc = __fadd_rn(acc, __fmul_rn(fx[m + 1], __fsub_rn(pc, p[m + 2])));
+                        acc = __fadd_rn(acc, __fmul_rn(fy[m], __fsub_rn(pc, lo_j[m * 256])));
+                        acc = __fadd_rn(acc, __fmul_rn(fy[4 + m], __fsub_rn(pc, hi_j[m * 256])));
+                        acc = __fadd_rn(acc, __fmul_rn(fz[m], __fsub_rn(pc, lo_k[m * 256])));
+                        a[m] = __fadd_rn(acc, __fmul_rn(fz[4 + m], __fsub_rn(pc, hi_k[m * 256])));
+                    }
+                }
+                div_rn4(a, hhd);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    ap[s * 4 + m] = a[m];
+                    pAp[s] = __fma_rn((double)p[m + 1], (double)a[m], pAp[s]);   // the product of two floats is exact
+                }
+                if (kWide) {
+                    int cells;
+                    const int t = first_cell(T, cells);
+#pragma unroll
+                    for (int m = 0; m < 4; ++m)
+                        if (m < cells) S.cg_Ap[t + m * n * n] = a[m];
+                    stash(q, pAp);
+                }
+            }
+            if (!kWide) stash(g, pAp);
+            ok = exchange<1, NT>(team, nt, step, red, tsum, sums, bad, [] {}, [&](const double (&tot)[1]) {
+                Ls.pAp = tot[0];
+                Ls.alpha = __double2float_rn(quotient(Ls.rz, tot[0]));
+            });
+            if (!ok) break;
+            const float alpha = Ls.alpha;
+            // x += alpha p, r -= alpha A p, z = D r; z of the shared faces goes out; r.r and r.z
+            double part[2 * QR];
+            ++pub;
+#pragma unroll (kWide ? 2 : QR)
+            for (int turn = 0; turn < turns; ++turn) {
+                const int s = kWide ? 0 : turn, q = G * turn + g;
+                part[s] = part[QR + s] = 0.0;
+                if (q >= nt) continue;
+                float d[4], z4[4];
+                diag(tt[q], s, d);
+                const float* core = sm + q * 1024 + lt;
+                float* x = sm + X + q * 1024 + lt;
+                if constexpr (kWide) {
+                    int cells;
+                    const int t = first_cell(tt[q], cells), nn = n * n;
+                    float xv[4];
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        const bool in = m < cells;
+                        r[m] = in ? S.cg_r[t + m * nn] : 0.0f;
+                        ap[m] = in ? S.cg_Ap[t + m * nn] : 0.0f;
+                        xv[m] = in ? S.p[t + m * nn] : 0.0f;
+                    }
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        r[m] = __fsub_rn(r[m], __fmul_rn(alpha, ap[m]));
+                        if (m < cells) {
+                            S.cg_r[t + m * nn] = r[m];
+                            S.p[t + m * nn] = __fadd_rn(xv[m], __fmul_rn(alpha, core[m * 256]));
+                        }
+                    }
+                }
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const int e = s * 4 + m;
+                    if (kKeepX)
+                        xr[e] = __fadd_rn(xr[e], __fmul_rn(alpha, pr[e]));
+                    else if (!kWide)
+                        x[m * 256] = __fadd_rn(x[m * 256], __fmul_rn(alpha, core[m * 256]));
+                    if (!kWide) r[e] = __fsub_rn(r[e], __fmul_rn(alpha, ap[e]));
+                    z4[m] = __fmul_rn(d[m], r[e]);
+                    part[s] = __fma_rn((double)r[e], (double)r[e], part[s]);
+                    part[QR + s] = __fma_rn((double)r[e], (double)z4[m], part[QR + s]);
+                }
+                post(tt[q], z4, team.base | (pub & 0x3ffu));
+                if (kWide) stash(q, part);
+            }
+            if (!kWide) stash(g, part);
+            {
+                ok = exchange<2, NT>(team, nt, step, red, tsum, sums, bad, [&] { fetch(team.base | (pub & 0x3ffu)); },
+                                     [&](const double (&tot)[2]) {
+                                         // the classic test, then beta (update_scalars)
+                                         const double rr = tot[0];
+                                         const bool above = rr > Ls.atol_sq, finite = isfinite(rr);
+                                         Ls.beta = above ? __double2float_rn(quotient(tot[1], Ls.rz)) : 0.0f;
+                                         Ls.rz = tot[1];
+                                         Ls.rr = rr;
+                                         Ls.iters = kit;
+                                         if (!finite) Ls.status |= HF_SCENE_NONFINITE;
+                                         Ls.live = above && finite && kit < Ls.maxit;
+                                         if (!Ls.live && above && finite) Ls.status |= HF_SCENE_PRESSURE_MAXITER;
+                                     });
+                if (!ok) break;
+                beta = Ls.beta;
+                live = Ls.live;
+            }
+        }
+        // ------------------------------------------------------------- x back, projection of the faces (grid.py:140-153)
+        if (ok) {
+            ++pub;
+#pragma unroll QR
+            for (int turn = 0; turn < turns; ++turn) {
+                const int s = kWide ? 0 : turn, q = G * turn + g;
+                if (q >= nt) continue;
+                float x4[4];
+                int cells;
+                const int t = first_cell(tt[q], cells);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    float& x = sm[X + q * 1024 + m * 256 + lt];
+                    if (kKeepX) x = xr[s * 4 + m];
+                    if (kWide) x = m < cells ? S.p[t + m * n * n] : 0.0f;
+                    x4[m] = x;
+                }
+                post(tt[q], x4, team.base | (pub & 0x3ffu));
+            }
+            __syncthreads();
+            if (warp >= kPollWarps) fetch(team.base | (pub & 0x3ffu));
+            take(team.base | (pub & 0x3ffu), [&](float& pb, float v) { pb = v; });
+            ok = !__syncthreads_or(bad);
+            if (bl.jobs > 1 && threadIdx.x == 0) {
+                asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ws.arrive + job) : "memory");
+                left = job;
+                left_nb = J.z;
+            }
+        }
+        if (ok) {
+            float *u = S.u[par ^ 1], *v = S.v[par ^ 1], *w = S.w[par ^ 1];
+            const float dtr = (float)(dt_d / S.rho);
+            for (int q = g; q < nt; q += G) {
+                const BrickTile& T = tt[q];
+                const TileItem it{0, T.i0, T.j0, T.k0};
+                auto at = [&](int o) { return o < X ? o + X : o; };   // the x of another tile of the block, or the halo
+                const int core = X + q * 1024 + lt;
+                const float* lo_j = sm + (row == 0 ? at(T.nb[2]) + lane : core - 32);
+                const float* lo_k = sm + (lane == 0 ? at(T.nb[4]) + row * 32 : core - 1);
+                float below = sm[at(T.nb[0]) + lt];
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const Cell cl = tile_cell(it, n, lt, m);
+                    const float pc = sm[core + m * 256];
+                    if (cl.ok) {
+                        if (!kWide) S.p[cl.t] = pc;
+                        const int i = cl.i, j = cl.j, k = cl.k;
+                        int f = uidx_(n, i, j, k);
+                        u[f] = i == 0 ? 0.0f : __fsub_rn(u[f], __fdiv_rn(__fmul_rn(dtr, __fsub_rn(pc, below)), h));
+                        f = vidx_(n, i, j, k);
+                        v[f] = j == 0 ? 0.0f : __fsub_rn(v[f], __fdiv_rn(__fmul_rn(dtr, __fsub_rn(pc, lo_j[m * 256])), h));
+                        f = widx_(n, i, j, k);
+                        w[f] = k == 0 ? 0.0f : __fsub_rn(w[f], __fdiv_rn(__fmul_rn(dtr, __fsub_rn(pc, lo_k[m * 256])), h));
+                        if (i == n - 1) u[uidx_(n, n, j, k)] = 0.0f;
+                        if (j == n - 1) v[vidx_(n, i, n, k)] = 0.0f;
+                        if (k == n - 1) w[widx_(n, i, j, n)] = 0.0f;
+                    }
+                    below = pc;
+                }
+            }
+        }
+        __syncthreads();
+        if (leader && threadIdx.x == 0) write_stats(S, Ls, false, !ok, par);
+        __syncthreads();
+    }
+    // the last block to leave prepares the next launch: another launch number, no error, no arrivals
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(ws.brick + 1, 1u) == gridDim.x - 1) {
+            if (bl.jobs > 1)
+                for (int q = 0; q < bl.jobs; ++q) ws.arrive[q] = 0;
+            ws.brick[1] = 0;
+            ws.brick[2] = 0;
+            ws.brick[0] = launch + 1;
+        }
+    }
+}
+
+const void* brick_kernel(const BrickLaunch& bl, int* threads) {
+    // the small variants keep every tile's fractions in a box (launch_brick passes fewer boxes where they do not fit)
+    const int tiles = bl.boxes < bl.tiles && bl.tiles <= kBrickMaxTiles ? kBrickMaxTiles : bl.tiles;
+    *threads = tiles <= 2 ? 512 : tiles <= 4 ? 1024 : 768;
+    if (tiles <= 2) return (const void*)k_brick<2, 1>;
+    if (tiles <= 4) return (const void*)k_brick<4, 1>;
+    if (tiles <= 6) return (const void*)k_brick<3, 2>;
+    if (tiles <= 9) return (const void*)k_brick<3, 3>;
+    if (tiles <= kBrickMaxTiles) return (const void*)k_brick<3, 5>;
+    return (const void*)k_brick<3, 0>;
+}
+
+size_t brick_smem(const BrickLaunch& bl) {
+    const size_t per_tile = bl.tiles <= kBrickMaxTiles ? 2048 : 1024;
+    return (bl.tiles * per_tile + (size_t)bl.pages * 1024 + (size_t)bl.boxes * kFaceBox) * sizeof(float);
+}
+
+int brick_box_bytes() { return kFaceBox * (int)sizeof(float); }
+
+int brick_set_wait_limit(unsigned long long limit_ns, int absent_block) {
+    if (cudaMemcpyToSymbol(c_wait_limit_ns, &limit_ns, sizeof limit_ns) != cudaSuccess) return HF_ERR_CUDA;
+    if (cudaMemcpyToSymbol(c_absent_block, &absent_block, sizeof absent_block) != cudaSuccess) return HF_ERR_CUDA;
+    return HF_OK;
+}
+
+}  // namespace hf

@@ -31,26 +31,14 @@
 //               TMA (cp.async.bulk.tensor) instead of gathered; x, r and D stay in registers.
 #include <cuda.h>
 
-#include "hf_device.cuh"
-#include "hf_kernels.cuh"
+#include "hf_cg.cuh"
 
 namespace hf {
 
-constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;   // 2 s
-// Limit of every bounded wait of the CG kernels (grid and lane barriers, TMA copies), and the block that does not
-// arrive at the first grid barrier of each persistent CG launch (-1: none).  The defaults are what every solve uses;
-// hf_set_wait_limit changes both, so that a test can make a barrier's wait run out on purpose and check that the
-// kernel reports HF_SCENE_BARRIER_TIMEOUT and returns with the context usable.
-__constant__ unsigned long long c_wait_limit_ns = kBarrierTimeoutNs;
-__constant__ int c_absent_block = -1;
 // Components one group_sum / scene_sums call reduces at most: 3 inner products per tile x 3 tiles of a 256-thread
 // group (the resident variants' set-up).  Every CG kernel's `red` holds kRedComps x 32 doubles (one per warp).
 constexpr int kRedComps = 9;
 constexpr int kMaxCorrections = 2;   // restarts of one solve by the outer defect correction
-
-__device__ __forceinline__ int uidx_(int n, int i, int j, int k) { return (i * n + j) * n + k; }
-__device__ __forceinline__ int vidx_(int n, int i, int j, int k) { return (i * (n + 1) + j) * n + k; }
-__device__ __forceinline__ int widx_(int n, int i, int j, int k) { return (i * n + j) * (n + 1) + k; }
 
 // Barrier of nblocks blocks (the grid, or one lane of it) with a bounded wait.  Thread 0 publishes the block's writes with a release reduction (cumulative over
 // the writes the block's threads made before __syncthreads) and polls with acquire loads.  Returns false (in every
@@ -76,26 +64,39 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned& epoch, int
     return *(volatile int*)err == 0;
 }
 
-// Sum of a scene's partials (item c, component comp[q] at buf[comp[q] * cs + c]: component-major, so that a warp's
-// loads of one component are contiguous) in a fixed tree: the first 256 threads stride over the items in order, warp
-// butterfly, then 8 warps in order.  Every block computing it obtains the same bits.  cs is the plan's tile count for
-// the tile partials (three components, see part_idx) and 0 for the per-chunk rhs sums (one component).
+// Sum of a scene's partials (item c, component comp[q] at buf[comp[q] * cs + c]: component-major) in a fixed tree: every
+// one of the first 256 threads adds its items in order, warp butterfly, then 8 warps in order.  Every block computing it
+// obtains the same bits.  Tile partials (cs: the plan's tile count): thread u adds the tiles of unit u (unit_first) when
+// the scene is one that the on-chip solve takes; of a larger scene (whose runs of 16 tiles and more would be as many
+// dependent round trips), and of the per-chunk rhs sums (cs = 0, one component), thread t adds items t, t + 256, ...
+struct Run {
+    int first, end, step;
+};
+
+// the items of [b, e) that this thread adds
+__device__ __forceinline__ Run thread_run(int b, int e, int cs) {
+    const int t = threadIdx.x, T = e - b, units = unit_count(T);
+    if (cs == 0 || T > kUnits * kBrickWideTiles) return Run{b + t, t < kThreads ? e : b, kThreads};
+    if (t >= units) return Run{b, b, 1};
+    return Run{b + unit_first(T, units, t), b + unit_first(T, units, t + 1), 1};
+}
+
 template <int K, int U = 4>
 __device__ __forceinline__ void scene_sums(const double* __restrict__ buf, int b, int e, const int (&comp)[K],
                                            double (&tot)[K], double* red, int cs) {
     static_assert(K <= kRedComps, "red holds kRedComps components");
 #pragma unroll
     for (int q = 0; q < K; ++q) tot[q] = 0.0;
-    if (threadIdx.x < kThreads) {
-        // a thread's partials c = b + t, b + t + 256, ... are added in that order; U at a time are loaded (an absent
-        // one as +0.0, which leaves a sum that started at +0.0 unchanged) before they are added, so their L2 round
-        // trips overlap instead of each waiting for the previous addition
-        for (int c = b + threadIdx.x; c < e; c += U * kThreads) {
+    const Run run = thread_run(b, e, cs);
+    if (run.first < run.end) {
+        // U items at a time are loaded (an absent one as +0.0, which leaves a sum that started at +0.0 unchanged) before
+        // they are added, so their L2 round trips overlap instead of each waiting for the previous addition
+        for (int c = run.first; c < run.end; c += U * run.step) {
             double v[U][K];
 #pragma unroll
             for (int u = 0; u < U; ++u)
 #pragma unroll
-                for (int q = 0; q < K; ++q) v[u][q] = c + u * kThreads < e ? buf[comp[q] * cs + c + u * kThreads] : 0.0;
+                for (int q = 0; q < K; ++q) v[u][q] = c + u * run.step < run.end ? buf[comp[q] * cs + c + u * run.step] : 0.0;
 #pragma unroll
             for (int u = 0; u < U; ++u)
 #pragma unroll
@@ -141,12 +142,13 @@ __device__ __forceinline__ void group_sums(const double* __restrict__ buf, const
             double acc[K];
 #pragma unroll
             for (int k = 0; k < K; ++k) acc[k] = 0.0;
-            for (int c = b + lt; c < e; c += 4 * kThreads) {
+            const Run run = thread_run(b, e, cs);
+            for (int c = run.first; c < run.end; c += 4 * run.step) {
                 double v[4][K];
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
 #pragma unroll
-                    for (int k = 0; k < K; ++k) v[u][k] = c + u * kThreads < e ? buf[comp[k] * cs + c + u * kThreads] : 0.0;
+                    for (int k = 0; k < K; ++k) v[u][k] = c + u * run.step < run.end ? buf[comp[k] * cs + c + u * run.step] : 0.0;
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -316,22 +318,6 @@ __device__ __forceinline__ void unit_sums(const double* __restrict__ buf, int un
         for (int w = 0; w < kThreads / 32; ++w) s += red[c * 32 + w];
         tot[c] = s;
     }
-}
-
-// cell m (0..3) of thread lt in a tile
-struct Cell {
-    int t, i, j, k;
-    bool ok;
-};
-
-__device__ __forceinline__ Cell tile_cell(const TileItem& ti, int n, int lt, int m) {
-    Cell c;
-    c.i = ti.i0 + m;
-    c.j = ti.j0 + (lt >> 5);
-    c.k = ti.k0 + (lt & 31);
-    c.ok = c.i < n && c.j < n && c.k < n;
-    c.t = (c.i * n + c.j) * n + c.k;
-    return c;
 }
 
 // Search direction at cell t for iteration k: p_k = z + beta p_{k-1} (warp's _cg_kernel_2), or z at k = 1.
@@ -514,54 +500,6 @@ __device__ __forceinline__ void project_cell(const hf_scene& S, float* u, float*
     if (k == n - 1) w[widx_(n, i, j, n)] = 0.0f;
 }
 
-// Per-block copy of a scene's CG scalars; every block derives them from the same partial sums, so all copies agree.
-struct LocalScene {
-    double rz, atol_sq, bb, rr, pAp, mean;
-    double true_rr;             // fp64 |b - A x|^2 of the outer defect correction (-1: not formed)
-    float alpha, beta;
-    int live, iters, maxit, status;
-    int kbase;                  // iterations before the last restart by the defect correction
-    int corrections;            // restarts so far
-    int dc;                     // the true residual is still to be checked (HF_FLAG_DEFECT_CORRECTION)
-};
-
-__device__ __forceinline__ void init_scalars(LocalScene& L, const hf_scene& S, bool heat, const double (&tot)[3], int N) {
-    const double tol = heat ? S.heat_tol : S.cg_tol;
-    double atol = tol * sqrt(tot[0]);
-    if (atol < tol) atol = tol;
-    if (atol < 1.0e-18) atol = 1.0e-18;
-    int maxit = heat ? S.heat_maxiter : S.cg_max_iter;
-    if (maxit <= 0) maxit = N;
-    L.maxit = maxit + (maxit & 1);   // iterations run in pairs
-    L.bb = tot[0];
-    L.rr = tot[1];
-    L.rz = tot[2];
-    L.atol_sq = atol * atol;
-    L.iters = 0;
-    L.beta = 0.0f;
-    L.alpha = 0.0f;
-    L.status = isfinite(tot[1]) ? 0 : HF_SCENE_NONFINITE;
-    L.live = tot[1] > L.atol_sq && isfinite(tot[1]) && L.maxit > 0;
-    L.true_rr = -1.0;
-    L.kbase = 0;
-    L.corrections = 0;
-    L.dc = (S.flags & HF_FLAG_DEFECT_CORRECTION) != 0;
-}
-
-// convergence test after phase B of iteration kit (warp: kernel_2 then the residual test)
-__device__ __forceinline__ bool update_scalars(LocalScene& L, bool heat, double rr, double rz, int kit) {
-    L.iters = kit;
-    const bool above = rr > L.atol_sq;
-    L.beta = above ? __double2float_rn(rz / L.rz) : 0.0f;
-    L.rz = rz;
-    L.rr = rr;
-    if (!isfinite(rr)) L.status |= HF_SCENE_NONFINITE;
-    const bool live = above && isfinite(rr) && kit < L.maxit;
-    if (!live && above && isfinite(rr)) L.status |= heat ? HF_SCENE_HEAT_MAXITER : HF_SCENE_PRESSURE_MAXITER;
-    L.live = live;
-    return live;
-}
-
 // True residual b - A x of one cell for the outer defect correction: the binary32 operator (grid.py:94-115 with the
 // binary32 h^2; heat.py:94-105 with the binary32 dt/h^2 and face diffusivities) applied with every product and sum in
 // fp64 to the binary32 vectors.
@@ -596,32 +534,6 @@ __device__ double true_residual_heat(const hf_scene& S, const float* __restrict_
         acc += (S.cell_flags[nbr[q]] & 1) ? kf * xc : kf * (xc - (double)x[nbr[q]]);
     }
     return b - (xc + c_dt * acc);
-}
-
-__device__ __forceinline__ void write_stats(const hf_scene& S, const LocalScene& L, bool heat, bool timed_out, int par) {
-    hf_scene_state* st = S.state;
-    if (heat) {
-        st->status = L.status | (timed_out ? HF_SCENE_BARRIER_TIMEOUT : 0);
-        st->heat_iters = L.iters;
-        st->heat_rr = L.rr;
-        st->heat_atol = sqrt(L.atol_sq);
-        st->heat_bb = L.bb;
-        st->heat_true_rr = L.true_rr;
-        st->total_heat_iters += L.iters;
-    } else {
-        st->status |= L.status | (timed_out ? HF_SCENE_BARRIER_TIMEOUT : 0);
-        st->pressure_iters = L.iters;
-        st->pressure_rr = L.rr;
-        st->pressure_atol = sqrt(L.atol_sq);
-        st->pressure_bb = L.bb;
-        st->pressure_true_rr = L.true_rr;
-        st->rhs_mean = L.mean;
-        st->total_pressure_iters += L.iters;
-        if (!timed_out) {
-            st->parity = par ^ 1;
-            st->substeps += 1;
-        }
-    }
 }
 
 // ============================================================================================ TMA staging
@@ -2344,7 +2256,7 @@ const void* pcg_resident_kernel(bool heat, int maxc, bool tma) {
 int set_wait_limit(unsigned long long limit_ns, int absent_block) {
     if (cudaMemcpyToSymbol(c_wait_limit_ns, &limit_ns, sizeof limit_ns) != cudaSuccess) return HF_ERR_CUDA;
     if (cudaMemcpyToSymbol(c_absent_block, &absent_block, sizeof absent_block) != cudaSuccess) return HF_ERR_CUDA;
-    return HF_OK;
+    return brick_set_wait_limit(limit_ns, absent_block);
 }
 
 size_t pcg_resident_smem(int groups, int maxc, bool tma, bool heat) {

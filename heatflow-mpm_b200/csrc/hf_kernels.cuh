@@ -32,8 +32,33 @@ struct Workspace {
                             // c * tiles + t (the single-reduction kernel: 5 components per 256-thread group)
     double* partB;          // [3 T] per-tile fp64 partials of the CG set-up and phase B (same layout)
     double* mean_part;      // [C] per-chunk fp64 sums of the pressure rhs
+    // the on-chip pressure solve (hf_brick.cu); absent from the workspace of a plan that only streams
+    unsigned* brick;        // launches so far, blocks that have left this launch, a wait of this launch gave up
+    unsigned* arrive;       // [S] members that have left a job
+    int4* jobs;             // [S] (scene, first block, blocks) in the blocks' common order
+    ulonglong2* mail;       // [blocks][2][kBrickWideTiles] 128-byte lines: every block's unit sums, two steps deep
+    unsigned long long* halo;   // [kHaloEntries T] (value, tag) words of the tiles' faces
     int tiles;              // T: tiles of the plan, the component stride of partA / partB
 };
+
+constexpr int kBrickMaxTiles = 15;   // tiles of an on-chip solve's block with r, A p and x on the chip at most,
+constexpr int kBrickWideTiles = 36;  // with p alone
+constexpr int kHaloEntries = 832;    // cells on the six faces of a tile, face by face
+
+// Launch of the on-chip pressure solve: `tiles` is the most that a block owns; halo pages of 1024 floats (for i faces, for
+// j faces, the rest for k faces) and boxes of face fractions follow p and x in shared memory.
+struct BrickLaunch {
+    int jobs, tiles, pages, i_pages, j_pages, boxes;
+    int4 job0;   // the only job, or unused (ws.jobs)
+};
+// the kernel for such blocks and its threads: (const hf_scene*, const TileItem*, double dt, Workspace, BrickLaunch), dynamic
+// shared memory brick_smem(...)
+const void* brick_kernel(const BrickLaunch& bl, int* threads);
+size_t brick_smem(const BrickLaunch& bl);
+int brick_box_bytes();
+int brick_set_wait_limit(unsigned long long limit_ns, int absent_block);
+// workspace bytes of a plan without the on-chip solve's part (streaming plans)
+size_t streaming_workspace_bytes(int num_scenes, int num_chunks, int num_tiles);
 
 // TMA descriptors of the tiled pressure stencil (resident CG): z, both search-direction buffers, alpha_f x (the u
 // lattice), and the cell-layout copies of alpha_f y and z.

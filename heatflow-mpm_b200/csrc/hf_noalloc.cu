@@ -44,7 +44,7 @@ ScratchLayout layout(int n, int C, int T) {
     L.tiles = o;
     o = up256(o + sizeof(hf::TileItem) * (size_t)T);
     L.ws = o;
-    L.ws_bytes = hf_workspace_bytes(1, C, T);
+    L.ws_bytes = hf::streaming_workspace_bytes(1, C, T);
     o = up256(o + L.ws_bytes);
     L.qzero = o;
     o = up256(o + sizeof(float) * NF);
@@ -184,7 +184,7 @@ extern "C" int hf_pressure_solve_noalloc(int n, double h, double rho, double dt,
 
     k_noalloc_setup<<<64, 256, 0, s>>>(rec, base, L, C, T, qx == nullptr);
     if (cudaGetLastError() != cudaSuccess) return hf::set_error(HF_ERR_CUDA, "hf_pressure_solve_noalloc: set-up launch failed");
-    // the workspace's offset tables (after the zeroing above): layout of hf_workspace_bytes(1, C, T)
+    // the workspace's offset tables (after the zeroing above): layout of streaming_workspace_bytes(1, C, T)
     hf_plan plan;
     std::memset(&plan, 0, sizeof plan);
     plan.num_scenes = 1;

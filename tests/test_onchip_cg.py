@@ -1,0 +1,58 @@
+"""The on-chip pressure solve (csrc/hf_brick.cu) against the streaming kernel: the same operations in the same order on the
+same values, so every field, iteration count and status is equal bit for bit.  Sizes at the edges of its variants: one
+tile and less, whole and ragged tiles, blocks of 1, 2, 4, 6, 9 and 15 tiles, p alone on the chip (beyond 15 tiles a block),
+the largest that fits and the first that does not."""
+import numpy as np
+import pytest
+
+from helpers import random_scene_inputs
+
+pytestmark = pytest.mark.gpu
+
+
+def _scenes(sizes, seed):
+    from heatflow_mpm.scene import DeviceScene
+    out = []
+    for i, n in enumerate(sizes):
+        spec, T0, uvw = random_scene_inputs(n, seed=seed + i)
+        sc = DeviceScene(spec)
+        sc.set_current("T", T0)
+        for nm, a in zip("uvw", uvw):
+            sc.set_current(nm, a)
+        out.append(sc)
+    return out
+
+
+def _equal(a, b):
+    for nm in ("T", "u", "v", "w"):
+        assert np.array_equal(a.current(nm).cpu().numpy(), b.current(nm).cpu().numpy()), (a.n, nm)
+    assert np.array_equal(a.p.cpu().numpy(), b.p.cpu().numpy()), a.n
+    sa, sb = a.read_state(), b.read_state()
+    assert (sa.pressure_iters, sa.heat_iters, sa.status) == (sb.pressure_iters, sb.heat_iters, sb.status)
+    assert (sa.pressure_rr, sa.pressure_bb, sa.rhs_mean) == (sb.pressure_rr, sb.pressure_bb, sb.rhs_mean)
+
+
+@pytest.mark.parametrize("n", [2, 5, 31, 32, 33, 50, 63, 70, 81, 96, 97, 111, 128, 130, 168, 169])
+def test_one_scene_equals_streaming(n):
+    from heatflow_mpm.scene import ScenePlan
+    (a,), (b,) = _scenes([n], 60), _scenes([n], 60)
+    chip, stream = ScenePlan([a]), ScenePlan([b], streaming_cg=True)
+    for plan in (chip, stream):
+        plan.prepare_statics()
+        for _ in range(2):
+            plan.substep(2e-3)
+    _equal(a, b)
+
+
+@pytest.mark.parametrize("sizes", [(20, 33, 47), (96, 96, 64, 64, 48, 40, 33, 32) * 2, (128, 24, 128, 57), (136, 40, 88)],
+                         ids=["side by side", "in turn", "large first", "p alone"])
+def test_batch_equals_streaming(sizes):
+    """Teams that share the blocks at the same time and one after another, over several launches of one plan."""
+    from heatflow_mpm.scene import ScenePlan
+    chip, stream = _scenes(sizes, 90), _scenes(sizes, 90)
+    for plan in (ScenePlan(chip), ScenePlan(stream, streaming_cg=True)):
+        plan.prepare_statics()
+        for _ in range(2):
+            plan.substep(2e-3)
+    for a, b in zip(chip, stream):
+        _equal(a, b)
