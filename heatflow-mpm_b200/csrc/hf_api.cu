@@ -39,14 +39,13 @@ struct DeviceInfo {
     int occ_heat = 0, occ_pressure = 0, occ_pressure_tma = 0;
     size_t smem_optin = 0;
     bool ready = false;
-    // occupancy of each resident variant [heat][tiles per group][tma][groups] (-1: not queried yet; the query also
+    // occupancy of the single-reduction pressure variant [tiles per group][groups] (-1: not queried yet; the query also
     // raises the kernel's dynamic shared-memory limit)
-    int res_occ[2][4][2][5];
-    int pipe_occ[4][5];   // the single-reduction pressure variant [tiles per group][groups] (-1: not queried yet)
-    bool brick_ready[2][hf::kBrickWideTiles + 1];  // the on-chip pressure solve's kernels whose shared-memory limit is raised
+    int pipe_occ[4][5];
+    bool brick_ready[3][hf::kBrickWideTiles + 1];  // the on-chip pressure solve's kernels whose shared-memory limit is raised
 };
 
-constexpr int kResGroupsMax[4] = {0, 4, 3, 2};   // 256-thread groups per block of the resident variant, by MAXC
+constexpr int kResGroupsMax[4] = {0, 4, 3, 2};   // 256-thread groups per block of the single-reduction variant, by MAXC
 
 std::mutex g_mu;
 DeviceInfo g_dev[64];
@@ -82,7 +81,6 @@ int device_info(DeviceInfo** out) {
         HF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "cudaDeviceGetAttribute");
         d.smem_optin = (size_t)optin;
         if (!d.coop) return fail(HF_ERR_DEVICE, "device does not support cooperative launches");
-        std::memset(d.res_occ, 0xff, sizeof d.res_occ);
         std::memset(d.pipe_occ, 0xff, sizeof d.pipe_occ);
         std::memset(d.brick_ready, 0, sizeof d.brick_ready);
         d.ready = true;
@@ -181,42 +179,7 @@ int encode_map(CUtensorMap* m, const float* base, int nk, int nj, int ni, int bk
 
 // The six TMA descriptors of a scene's tiled pressure stencil (order of hf::TileMaps): z and both search-direction
 // buffers with a one-cell halo, alpha_f x on its face lattice, alpha_f y and z in cell layout.
-static_assert(sizeof(hf::TileMaps) == 12 * sizeof(CUtensorMap), "TileMaps is twelve consecutive descriptors");
-
-// a 3-D byte array (k fastest) of dims (nk, nj, ni) with a box (bk, bj, bi): nk and bk multiples of 16
-int encode_map_u8(CUtensorMap* m, const uint8_t* base, int nk, int nj, int ni, int bk, int bj, int bi) {
-    if (!g_encode) {
-        CUtensorMap probe;
-        int rc = encode_map(&probe, reinterpret_cast<const float*>(base), 4, 1, 1, 4, 1, 1);   // loads the entry point
-        if (rc) return rc;
-    }
-    const cuuint64_t dims[3] = {(cuuint64_t)nk, (cuuint64_t)nj, (cuuint64_t)ni};
-    const cuuint64_t strides[2] = {(cuuint64_t)nk, (cuuint64_t)nk * nj};
-    const cuuint32_t box[3] = {(cuuint32_t)bk, (cuuint32_t)bj, (cuuint32_t)bi};
-    const cuuint32_t es[3] = {1, 1, 1};
-    CUresult r = g_encode(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t*>(base), dims, strides, box, es,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(HF_ERR_DEVICE, "cuTensorMapEncodeTiled (bytes) failed");
-    return HF_OK;
-}
-
-// The TMA descriptors of a scene's tiled heat stencil: the z / p boxes of the pressure geometry, the face
-// diffusivities x (face lattice, like alpha_f x), y (rows j0..j0+8 of the (n, n+1, n) face lattice) and z (cell-layout
-// copy), and the cell flags with a one-cell halo (k origin 16-byte aligned).  Needs n % 16 == 0 (byte rows).
-int encode_heat_maps(const hf_scene& sc, hf::TileMaps& m) {
-    const int n = sc.n;
-    int rc;
-    if ((rc = encode_map(&m.z, sc.cg_z, n, n, n, 40, 10, 6))) return rc;
-    if ((rc = encode_map(&m.p0, sc.cg_p[0], n, n, n, 40, 10, 6))) return rc;
-    if ((rc = encode_map(&m.p1, sc.cg_p[1], n, n, n, 40, 10, 6))) return rc;
-    if ((rc = encode_map(&m.hkx, sc.hkx, n, n, n + 1, 32, 8, 5))) return rc;
-    if ((rc = encode_map(&m.hky, sc.hky, n, n + 1, n, 32, 9, 4))) return rc;
-    if ((rc = encode_map(&m.hkzc, sc.hkzc, n, n, n, 36, 8, 4))) return rc;
-    if ((rc = encode_map(&m.t0, sc.T[0], n, n, n, 40, 10, 6))) return rc;
-    if ((rc = encode_map(&m.t1, sc.T[1], n, n, n, 40, 10, 6))) return rc;
-    return encode_map_u8(&m.flags, sc.cell_flags, n, n, n, 64, 10, 6);
-}
+static_assert(sizeof(hf::TileMaps) == 6 * sizeof(CUtensorMap), "TileMaps is six consecutive descriptors");
 
 int encode_scene_maps(const hf_scene& sc, CUtensorMap* m) {
     const int n = sc.n;
@@ -326,14 +289,14 @@ bool brick_schedule(const hf_plan* p, int sms, BrickSchedule& out) {
     return brick_schedule(p, sms, hf::kBrickMaxTiles, out) || brick_schedule(p, sms, hf::kBrickWideTiles, out);
 }
 
-// The on-chip pressure solve of a plan whose scenes all fit.  HF_OK after launching, -1 when it does not apply.
-int launch_brick(const hf_plan* p, DeviceInfo* d, double dt, void* stream) {
+// The on-chip solve of a plan whose scenes all fit.  HF_OK after launching, -1 when it does not apply.
+int launch_brick(const hf_plan* p, DeviceInfo* d, bool heat, double dt, void* stream) {
     if (!(p->options & HF_PLAN_MAPS_READY) || p->workspace_bytes < layout(p->num_scenes, p->num_chunks, p->num_tiles).total) return -1;
     BrickSchedule sched;
     if (!brick_schedule(p, d->sms, sched)) return -1;
     for (int s = 0; s < p->num_scenes; ++s) {
         const hf_scene& sc = p->scenes_host[s];
-        if ((sc.flags & HF_FLAG_ACTIVE) && (!sc.pdiag || !sc.cg_r || !sc.cg_Ap)) return -1;   // scratch of the larger variants
+        if ((sc.flags & HF_FLAG_ACTIVE) && (!sc.pdiag || !sc.hdiag || !sc.cg_r || !sc.cg_z || !sc.cg_Ap)) return -1;   // scratch of the larger variants
     }
     hf::BrickLaunch bl;
     std::memset(&bl, 0, sizeof bl);
@@ -349,10 +312,10 @@ int launch_brick(const hf_plan* p, DeviceInfo* d, double dt, void* stream) {
     // general tiles read the lattices
     const size_t room = d->smem_optin - (bl.tiles <= hf::kBrickMaxTiles ? 9 : 19) * 1024, base = hf::brick_smem(bl);
     if (base > room) return -1;
-    bl.boxes = std::min(bl.tiles, (int)((room - base) / hf::brick_box_bytes()));
+    bl.boxes = heat ? 0 : std::min(bl.tiles, (int)((room - base) / hf::brick_box_bytes()));
     int threads = 0;
-    const void* fn = hf::brick_kernel(bl, &threads);
-    bool& ready = d->brick_ready[bl.boxes < bl.tiles][bl.tiles];
+    const void* fn = hf::brick_kernel(bl, heat, &threads);
+    bool& ready = d->brick_ready[heat ? 2 : bl.boxes < bl.tiles][bl.tiles];
     if (!ready) {
         cudaFuncAttributes at;
         HF_CUDA(cudaFuncGetAttributes(&at, fn), "attributes (on-chip CG)");
@@ -369,9 +332,9 @@ int launch_brick(const hf_plan* p, DeviceInfo* d, double dt, void* stream) {
     return HF_OK;
 }
 
-// The resident variant for a plan with one active scene whose tiles fit one block per SM.  Returns HF_OK after
-// launching, or -1 when the scene does not fit (the caller falls back to the streaming kernel).
-int launch_resident(const hf_plan* p, DeviceInfo* d, bool heat, double dt, int s, void* stream) {
+// The single-reduction pressure solve of a plan with one active scene (n % 4 == 0) whose tiles fit one block per SM.
+// Returns HF_OK after launching, or -1 when it does not apply (the caller falls back to the classic solves).
+int launch_one(const hf_plan* p, DeviceInfo* d, double dt, int s, void* stream) {
     hf::Workspace ws = workspace(p);
     const hf_scene* scenes = static_cast<const hf_scene*>(p->scenes_dev);
     const hf::TileItem* tiles = static_cast<const hf::TileItem*>(p->tiles_dev);
@@ -380,50 +343,46 @@ int launch_resident(const hf_plan* p, DeviceInfo* d, bool heat, double dt, int s
     const int nt = t_hi - t_lo;
     const int G = nt < d->sms ? nt : d->sms;
     const int tpb = (nt + G - 1) / G;
-    // TMA-staged stencils: pressure with n % 4 == 0 (16-byte float rows), heat with n % 16 == 0 (16-byte flag rows)
-    const bool tma = !(p->options & HF_PLAN_NO_TMA) &&
-                     (heat ? (sc.n % 16 == 0 && sc.hkzc && sc.hkx && sc.hky && sc.cell_flags) : (sc.n % 4 == 0));
+    // its stencil boxes are staged by TMA (16-byte float rows) and its scratch vectors must exist
+    if ((p->options & HF_PLAN_NO_TMA) || sc.n % 4 != 0 || !sc.cg_r || !sc.cg_z || !sc.cg_Ap || !sc.hdiag || !sc.pdiag ||
+        !sc.cg_p[0] || !sc.cg_p[1])
+        return -1;
     const int want = (int)((p->options >> HF_PLAN_RES_TILES_SHIFT) & 3u);   // 0: the first that fits
-    // the single-reduction pressure solve (one grid barrier per iteration) when the plan asks for it, the stencil is
-    // staged and its scratch vectors exist
-    const bool pipe = !heat && tma && (p->options & HF_PLAN_SINGLE_REDUCTION_CG) && sc.cg_r && sc.cg_z && sc.cg_Ap &&
-                      sc.hdiag && sc.pdiag && sc.cg_p[0] && sc.cg_p[1];
-    if (!heat && !pipe) return -1;
-    // tiles per group: the fewest that fit; the single-reduction pressure kernel prefers three (two 256-thread groups
-    // of 128 registers per thread: its per-thread state does not fit the 80 registers of a 768-thread block)
-    const bool three_first = pipe && !want && tpb > 4;
+    // tiles per group: three first (two 256-thread groups of 128 registers per thread: the per-thread state does not fit
+    // the 80 registers of a 768-thread block), unless the block has few
+    const bool three_first = !want && tpb > 4;
     for (int mi = 0; mi < 3; ++mi) {
         const int m = want ? want + mi : (three_first ? 3 - mi : 1 + mi);
         if (m > 3) break;
         const int groups = (tpb + m - 1) / m;
         if (groups > kResGroupsMax[m]) continue;
-        // the single-reduction kernel publishes one set of partials per 256-thread group into buffers sized by tiles
-        if (pipe && G * groups > nt) continue;
-        const void* fn = pipe ? hf::pcg_one_kernel(m) : hf::pcg_resident_kernel(heat, m, tma);
-        const size_t smem = pipe ? hf::pcg_one_smem(groups, m) : hf::pcg_resident_smem(groups, m, tma, heat);
+        // one set of partials per 256-thread group into buffers sized by tiles
+        if (G * groups > nt) continue;
+        const void* fn = hf::pcg_one_kernel(m);
+        const size_t smem = hf::pcg_one_smem(groups, m);
         if (smem > d->smem_optin) continue;
-        int& occ = pipe ? d->pipe_occ[m][groups] : d->res_occ[heat][m][tma][groups];
+        int& occ = d->pipe_occ[m][groups];
         if (occ < 0) {
             if (smem > 48 * 1024)
                 HF_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attribute");
             int o = 0;
-            HF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, 256 * groups, smem), "occupancy (resident)");
+            HF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, 256 * groups, smem), "occupancy (single-reduction)");
             occ = o;
         }
         if (occ < 1) continue;
         hf::TileMaps maps;
         std::memset(&maps, 0, sizeof maps);
-        if (tma && (rc = heat ? encode_heat_maps(sc, maps) : encode_scene_maps(sc, &maps.z))) return rc;
+        if ((rc = encode_scene_maps(sc, &maps.z))) return rc;
         HF_CUDA(cudaMemsetAsync(ws.bar, 0, kHeadBytes, S(stream)), "cudaMemsetAsync(barrier)");
         void* args[] = {(void*)&scenes, (void*)&tiles, (void*)&t_lo, (void*)&t_hi, (void*)&dt, (void*)&ws, (void*)&maps};
         HF_CUDA(cudaLaunchCooperativeKernel(fn, dim3(G), dim3(256 * groups), args, smem, S(stream)),
-                "cooperative launch (resident CG)");
+                "cooperative launch (single-reduction CG)");
         return HF_OK;
     }
     return -1;
 }
 
-// Both CG solves of a plan.  One active scene: the resident variant where it fits.  Otherwise one launch of the
+// Both CG solves of a plan.  The on-chip solve where every active scene fits it.  Otherwise one launch of the
 // streaming kernel: the active scenes are cut, in table order, into groups of at most kGroupScenes scenes and
 // group_cells cells (default kGroupCells: a group's CG vectors stay in L2), solved by the lanes of the grid.
 int launch_pcg(const hf_plan* p, bool heat, double dt, void* stream) {
@@ -441,16 +400,14 @@ int launch_pcg(const hf_plan* p, bool heat, double dt, void* stream) {
             correction = correction || (p->scenes_host[s].flags & HF_FLAG_DEFECT_CORRECTION);
         }
     if (total != p->num_tiles) return fail(HF_ERR_ARG, "plan changed since hf_plan_upload");
-    if (!correction && !(p->options & HF_PLAN_STREAMING_CG)) {
-        const bool one_reduction = !heat && (p->options & HF_PLAN_SINGLE_REDUCTION_CG);
-        if (nactive == 1 && (heat ? !(p->options & HF_PLAN_STREAMING_HEAT) : one_reduction)) {
-            rc = launch_resident(p, d, heat, dt, last, stream);
+    if (nactive > 0 && !correction && !(p->options & HF_PLAN_STREAMING_CG) &&
+        !(heat && nactive == 1 && (p->options & HF_PLAN_STREAMING_HEAT))) {
+        if (!heat && nactive == 1 && (p->options & HF_PLAN_SINGLE_REDUCTION_CG)) {
+            rc = launch_one(p, d, dt, last, stream);
             if (rc != -1) return rc;
         }
-        if (!heat && nactive > 0) {
-            rc = launch_brick(p, d, dt, stream);
-            if (rc != -1) return rc;
-        }
+        rc = launch_brick(p, d, heat, dt, stream);
+        if (rc != -1) return rc;
     }
     static thread_local hf::GroupTable gt;   // 16 KB: kept off the stack; the launch copies it
     gt.count = 0;

@@ -1,8 +1,8 @@
-// hf_brick.cu -- the pressure solve with the CG state on the chip, one scene per team of blocks.
+// hf_brick.cu -- the CG solves with their state on the chip, one scene per team of blocks.
 //
-// Same system, arithmetic and reduction trees as the streaming kernel (hf_cg.cu): mean removal, Jacobi-preconditioned CG
-// warm-started from p, projection, end of the substep (grid.py:235-251, 94-153).  A team of blocks (one 512-thread block
-// per SM) owns a scene's tiles in contiguous runs of whole units; r, A p (and D) of a block's cells live in registers, p
+// Same systems, arithmetic and reduction trees as the streaming kernel (hf_cg.cu): the pressure solve -- mean removal,
+// Jacobi-preconditioned CG warm-started from p, projection, end of the substep (grid.py:235-251, 94-153) -- and the heat
+// solve (heat.py:198-210).  A team of blocks (one per SM) owns a scene's tiles in contiguous runs of whole units; r, A p (and D) of a block's cells live in registers, p
 // and x in shared memory, so an iteration moves only what blocks owe each other.  A plan of several scenes gives every
 // scene a team of its own and a place in the blocks' common order (BrickJobs, hf_api.cu); teams work side by side.
 //
@@ -250,7 +250,7 @@ __device__ __forceinline__ bool exchange(const Team& team, int nt, unsigned& ste
 // cell's faces, and other tiles read it back.
 // Q = 0, for large scenes: only p stays on the chip.  r, A p and x are read and written where they are used, by the thread
 // that owns the cell (28 bytes of L2 traffic per cell and iteration; the streaming kernel moves 60 and p's halo from HBM).
-template <int G, int Q>
+template <int G, int Q, bool HEAT>
 __global__ void __launch_bounds__(256 * G, 1)
     k_brick(const hf_scene* __restrict__ scenes, const TileItem* __restrict__ tiles, double dt_d, Workspace ws, BrickLaunch bl) {
     constexpr bool kWide = Q == 0;
@@ -269,6 +269,7 @@ __global__ void __launch_bounds__(256 * G, 1)
     __shared__ float kface[2 * 32];               // values of the run's two k faces on their way out
     __shared__ double sums[3][8];
     __shared__ LocalScene Ls;
+    __shared__ hf_scene Ss;
     __shared__ float dtab[8];
     __shared__ int s_count[5];                    // i planes, j slots, k columns, rows, face boxes in use
     const int g = threadIdx.x >> 8, lt = threadIdx.x & 255, lane = lt & 31, row = lt >> 5, warp = threadIdx.x >> 5;
@@ -282,10 +283,14 @@ __global__ void __launch_bounds__(256 * G, 1)
     for (int job = 0; job < bl.jobs; ++job) {
         const int4 J = bl.jobs == 1 ? bl.job0 : ws.jobs[job];   // scene, first block, blocks
         if ((int)blockIdx.x < J.y || (int)blockIdx.x >= J.y + J.z) continue;
-        const hf_scene& S = scenes[J.x];
+        // the scene's record in shared memory: its pointers are fetched again and again, and a trip to L2 before every access
+        // made the set-up and the projection several times slower
+        for (int w = threadIdx.x; w < (int)(sizeof(hf_scene) / sizeof(int)); w += 256 * G)
+            reinterpret_cast<int*>(&Ss)[w] = reinterpret_cast<const int*>(scenes + J.x)[w];
+        const hf_scene& S = Ss;
         const bool leader = (int)blockIdx.x == J.y;
         if (__syncthreads_or(*(volatile int*)err)) {   // a wait gave up earlier in this launch: the scene stays unsolved
-            if (leader && threadIdx.x == 0) S.state->status |= HF_SCENE_BARRIER_TIMEOUT;
+            if (leader && threadIdx.x == 0) S.state->status = (HEAT ? 0 : S.state->status) | HF_SCENE_BARRIER_TIMEOUT;
             continue;
         }
         Team team;
@@ -299,7 +304,7 @@ __global__ void __launch_bounds__(256 * G, 1)
         team.post = ws.mail + (size_t)blockIdx.x * 2 * kLines * 8;
         {
             // the owner of unit t and the unit's place among its units
-            const int t = (int)threadIdx.x < team.units ? threadIdx.x : 0, o = (int)(((long long)(t + 1) * J.z - 1) / team.units);
+            const int t = (int)threadIdx.x < team.units ? threadIdx.x : 0, o = ((t + 1) * J.z - 1) / team.units;
             team.poll = ws.mail + ((size_t)(J.y + o) * 2 * kLines + t - unit_first(team.units, J.z, o)) * 8;
         }
         team.base = launch << 20 | (unsigned)job << 10;
@@ -309,6 +314,9 @@ __global__ void __launch_bounds__(256 * G, 1)
         const int n = S.n, par = S.state->parity;
         const float h = (float)S.h, hh = __fmul_rn(h, h);
         const DivBy hhd = div_by(hh);
+        const float c_dt = __fdiv_rn((float)dt_d, hh);
+        float* const xg = HEAT ? S.T[par ^ 1] : S.p;
+        float* const Dg = HEAT ? S.hdiag : S.pdiag;
         const int ti = (n + kTI - 1) / kTI, tj = (n + kTJ - 1) / kTJ, tk = (n + kTK - 1) / kTK;
 
         // ------------------------------------------------------------------------------------ the block's tiles
@@ -326,7 +334,7 @@ __global__ void __launch_bounds__(256 * G, 1)
             t.slot = (tb + c) * kHaloEntries;
             t.remote = 0;
             t.face = -1;
-            t.unit = it.i0 + kTI <= n && it.j0 + kTJ <= n && it.k0 + kTK <= n;
+            t.unit = !HEAT && it.i0 + kTI <= n && it.j0 + kTJ <= n && it.k0 + kTK <= n;
             const bool there[6] = {it.i0 > 0, it.i0 / kTI + 1 < ti, it.j0 > 0, it.j0 / kTJ + 1 < tj, it.k0 > 0, it.k0 / kTK + 1 < tk};
             const int away[6] = {-tk, tk, -tk * ti, tk * ti, -1, 1};
             // offsets within the neighbour's core, and within the tile's own (domain faces: the cell itself)
@@ -370,8 +378,9 @@ __global__ void __launch_bounds__(256 * G, 1)
         }
         // the pressure rhs mean (grid.py:238-241) from the divergence stage's chunk sums: 256 threads in strides, warp
         // butterfly, 8 warps in order
-        float mean;
-        {
+        float mean = 0.0f;
+        __syncthreads();
+        if (!HEAT) {
             double m = 0.0;
             if (threadIdx.x < kThreads)
                 for (int c = ws.chunk_begin[J.x] + threadIdx.x; c < ws.chunk_begin[J.x + 1]; c += kThreads) m += ws.mean_part[c];
@@ -460,6 +469,51 @@ __global__ void __launch_bounds__(256 * G, 1)
                 apply(sm[place(r)], await(r, tag, ld_relaxed(ws.halo + rows[r].x + lane)));
         };
 
+        // the first of a tile's four cells, and which of them the domain has
+        auto first_cell = [&](const BrickTile& T, int& cells) {
+            const int j = T.j0 + row, k = T.k0 + lane;
+            cells = j < n && k < n ? min(4, n - T.i0) : 0;
+            return (T.i0 * n + j) * n + k;
+        };
+        // Face coefficients around two cells (i, j, k) and (i + 1, j, k) from the lattices: x faces i .. i + 2, low and high
+        // y and z faces; 0 where a face has no cell on one side, so that its term drops out.  Two cells at a time: their
+        // loads are in flight together and fit the registers.  (Taking the z neighbours from the next lane saved a third
+        // of the loads and made the set-up a quarter slower: the shuffles wait for the loads one by one.)
+        const int nn = n * n;
+        const float* const cx = HEAT ? S.hkx : S.ax;
+        const float* const cy = HEAT ? S.hky : S.ay;
+        const float* const cz = HEAT ? S.hkz : S.az;
+        auto coefficients = [&](int i, int j, int k, float (&fx)[3], float (&fy)[4], float (&fz)[4]) {
+            const bool in = j < n && k < n;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) fx[a] = in && i + a > 0 && i + a < n ? cx[uidx_(n, i + a, j, k)] : 0.0f;
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                const bool im = in && i + a < n;
+                fy[a] = im && j > 0 ? cy[vidx_(n, i + a, j, k)] : 0.0f;
+                fy[2 + a] = im && j < n - 1 ? cy[vidx_(n, i + a, j + 1, k)] : 0.0f;
+                fz[a] = im && k > 0 ? cz[widx_(n, i + a, j, k)] : 0.0f;
+                fz[2 + a] = im && k < n - 1 ? cz[widx_(n, i + a, j, k + 1)] : 0.0f;
+            }
+        };
+        // the cell values (or flags) of the same two cells and their neighbours: i - 1 .. i + 2, low and high j and k; 0
+        // outside the domain
+        auto around = [&](const auto* from, int i, int j, int k, auto (&vi)[4], auto (&vj)[4], auto (&vk)[4]) {
+            const bool in = j < n && k < n;
+            const int t = (i * n + j) * n + k;
+#pragma unroll
+            for (int a = 0; a < 4; ++a) vi[a] = in && i + a > 0 && i + a <= n ? from[t + (a - 1) * nn] : 0;
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                const bool im = in && i + a < n;
+                vj[a] = im && j > 0 ? from[t + a * nn - n] : 0;
+                vj[2 + a] = im && j < n - 1 ? from[t + a * nn + n] : 0;
+                vk[a] = im && k > 0 ? from[t + a * nn - 1] : 0;
+                vk[2 + a] = im && k < n - 1 ? from[t + a * nn + 1] : 0;
+            }
+        };
+        // one face's term of the stencil; heat: a fixed neighbour enters as kappa_f x_c (heat.py:55-91)
+        auto term = [](float c, bool fixed, float xc, float xn) { return __fmul_rn(c, HEAT && fixed ? xc : __fsub_rn(xc, xn)); };
         // the warp's sums of K components of its tiles (one: q, wide; else the group's) go to red
         auto stash = [&](int q, auto& part) {
             constexpr int N = (int)(sizeof(part) / sizeof(double)), P = pow2_above(N);
@@ -472,8 +526,11 @@ __global__ void __launch_bounds__(256 * G, 1)
         // ------------------------------------------------------------------------------------ set-up
         float r[4 * QR], ap[4 * QR], dg[kKeepD ? 4 * QR : 1], xr[kKeepX ? 4 * QR : 1], pr[kKeepX ? 4 * QR : 1];
         const int turns = kWide ? (nt - g + G - 1) / G : Q;   // of the loops over a group's tiles; unrolled unless wide
+        // heat: byte m: which of cell m's neighbours (in the faces' order) and, bit 6, the cell itself are fixed
+        unsigned fixed[HEAT ? QR : 1];
         {
-            // x0 = p, b = rhs - mean, D (k_jacobi), r0 = b - A x0, z0 = D r0; a tile with a fraction other than 1 is general
+            // x0, b, D, r0 = b - A x0, z0 = D r0; pressure: x0 = p, b = rhs - mean, and a tile with a fraction other than 1
+            // is general; heat: x0 = the advected T, b = hrhs
             double part[3 * QR];
 #pragma unroll QR
             for (int turn = 0; turn < turns; ++turn) {
@@ -481,62 +538,78 @@ __global__ void __launch_bounds__(256 * G, 1)
                 part[s] = part[QR + s] = part[2 * QR + s] = 0.0;
                 float z4[4];
                 if (q < nt) {
-                    const TileItem it{0, tt[q].i0, tt[q].j0, tt[q].k0};
+                    const int j = tt[q].j0 + row, k = tt[q].k0 + lane;
                     bool one = true;
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        const int e = s * 4 + m;
-                        const Cell cl = tile_cell(it, n, lt, m);
-                        float xc = 0.0f, z = 0.0f;
-                        r[e] = ap[e] = 0.0f;
-                        if (kKeepD) dg[e] = 0.0f;
-                        if (cl.ok) {
-                            const int t = cl.t, nn = n * n;
-                            const bool in[6] = {cl.i > 0, cl.i < n - 1, cl.j > 0, cl.j < n - 1, cl.k > 0, cl.k < n - 1};
-                            const int away[6] = {-nn, nn, -n, n, -1, 1};
-                            const float* at[6] = {S.ax + uidx_(n, cl.i, cl.j, cl.k), S.ax + uidx_(n, cl.i + 1, cl.j, cl.k),
-                                                  S.ay + vidx_(n, cl.i, cl.j, cl.k), S.ay + vidx_(n, cl.i, cl.j + 1, cl.k),
-                                                  S.az + widx_(n, cl.i, cl.j, cl.k), S.az + widx_(n, cl.i, cl.j, cl.k + 1)};
-                            float af[6], xn[6];
-                            xc = S.p[t];
+                    for (int m0 = 0; m0 < 4; m0 += 2) {
+                        const int i0 = tt[q].i0 + m0, t0 = (i0 * n + j) * n + k;
+                        float fx[3], fy[4], fz[4], xi[4], xj[4], xk[4], bv[2];
+                        int gi[4] = {}, gj[4] = {}, gk[4] = {};
+                        coefficients(i0, j, k, fx, fy, fz);
+                        around(xg, i0, j, k, xi, xj, xk);
+                        if (HEAT) around(S.cell_flags, i0, j, k, gi, gj, gk);
+                        const bool ok2[2] = {j < n && k < n && i0 < n, j < n && k < n && i0 + 1 < n};
 #pragma unroll
-                            for (int f = 0; f < 6; ++f) {
-                                af[f] = __ldg(at[f]);
-                                xn[f] = S.p[in[f] ? t + away[f] : t];
-                            }
-                            float bv = S.rhs[t];
-                            if (mean != 0.0f) {
-                                bv = __fsub_rn(bv, mean);
-                                S.rhs[t] = bv;
-                            }
-                            float sa = 0.0f, acc = 0.0f;
+                        for (int a = 0; a < 2; ++a) bv[a] = ok2[a] ? (HEAT ? S.hrhs : S.rhs)[t0 + a * nn] : 0.0f;
 #pragma unroll
-                            for (int f = 0; f < 6; ++f)
-                                if (in[f]) {
-                                    sa = __fadd_rn(sa, af[f]);
-                                    acc = __fadd_rn(acc, __fmul_rn(af[f], __fsub_rn(xc, xn[f])));
-                                    one = one && af[f] == 1.0f;
+                        for (int a = 0; a < 2; ++a) {
+                            const int m = m0 + a, e = s * 4 + m, i = i0 + a;
+                            const float xc = xi[a + 1];
+                            const float af[6] = {fx[a], fx[a + 1], fy[a], fy[2 + a], fz[a], fz[2 + a]};
+                            float sa = af[0];
+#pragma unroll
+                            for (int f = 1; f < 6; ++f) sa = __fadd_rn(sa, af[f]);
+                            const int mask = (gi[a] & 1) | (gi[a + 2] & 1) << 1 | (gj[a] & 1) << 2 | (gj[2 + a] & 1) << 3 |
+                                             (gk[a] & 1) << 4 | (gk[2 + a] & 1) << 5 | (gi[a + 1] & 1) << 6;
+                            if (HEAT) fixed[s] = m ? fixed[s] | (unsigned)mask << (8 * m) : (unsigned)mask;
+                            float acc = term(af[0], mask & 1, xc, xi[a]);
+                            acc = __fadd_rn(acc, term(af[1], mask & 2, xc, xi[a + 2]));
+                            acc = __fadd_rn(acc, term(af[2], mask & 4, xc, xj[a]));
+                            acc = __fadd_rn(acc, term(af[3], mask & 8, xc, xj[2 + a]));
+                            acc = __fadd_rn(acc, term(af[4], mask & 16, xc, xk[a]));
+                            acc = __fadd_rn(acc, term(af[5], mask & 32, xc, xk[2 + a]));
+                            float d = 0.0f, rv = 0.0f, z = 0.0f;
+                            if (ok2[a]) {
+                                if (mean != 0.0f) {
+                                    bv[a] = __fsub_rn(bv[a], mean);
+                                    S.rhs[t0 + a * nn] = bv[a];
                                 }
-                            const float d = __fdiv_rn(hh, maxf_(sa, 1.0e-12f)), rv = __fsub_rn(bv, __fdiv_rn(acc, hh));
-                            z = __fmul_rn(d, rv);
+                                if (HEAT) {   // k_heat_diag; identity rows on fixed cells
+                                    d = mask & 64 ? 1.0f : __fdiv_rn(1.0f, __fadd_rn(1.0f, __fmul_rn(c_dt, sa)));
+                                    rv = __fsub_rn(bv[a], mask & 64 ? xc : __fadd_rn(xc, __fmul_rn(c_dt, acc)));
+                                } else {      // k_jacobi
+                                    d = __fdiv_rn(hh, maxf_(sa, 1.0e-12f));
+                                    rv = __fsub_rn(bv[a], div_rn(acc, hhd));
+                                    one = one && (af[0] == 1.0f || i == 0) && (af[1] == 1.0f || i == n - 1) && (af[2] == 1.0f || j == 0) &&
+                                          (af[3] == 1.0f || j == n - 1) && (af[4] == 1.0f || k == 0) && (af[5] == 1.0f || k == n - 1);
+                                }
+                                z = __fmul_rn(d, rv);
+                                if (kWide) S.cg_r[t0 + a * nn] = rv;
+                                if (!kKeepD) Dg[t0 + a * nn] = d;
+                                part[s] += (double)bv[a] * (double)bv[a];
+                                part[QR + s] += (double)rv * (double)rv;
+                                part[2 * QR + s] += (double)rv * (double)z;
+                            }
                             r[e] = rv;
-                            if (kWide) S.cg_r[t] = rv;
+                            ap[e] = 0.0f;
                             if (kKeepD) dg[e] = d;
-                            else S.pdiag[t] = d;
-                            part[s] += (double)bv * (double)bv;
-                            part[QR + s] += (double)rv * (double)rv;
-                            part[2 * QR + s] += (double)rv * (double)z;
+                            z4[m] = z;
+                            if (kKeepX) {
+                                xr[e] = xc;
+                                pr[e] = z;
+                            } else if (!kWide) {
+                                sm[X + q * 1024 + m * 256 + lt] = xc;
+                            }
+                            sm[q * 1024 + m * 256 + lt] = z;
                         }
-                        z4[m] = z;
-                        if (kKeepX) {
-                            xr[e] = xc;
-                            pr[e] = z;
-                        } else if (!kWide) {
-                            sm[X + q * 1024 + m * 256 + lt] = xc;
-                        }
-                        sm[q * 1024 + m * 256 + lt] = z;
+                        asm volatile("" ::: "memory");   // the next two cells' loads stay behind
                     }
                     if (!one) tt[q].unit = 0;
+                    if (HEAT && kWide) {
+                        int cells;
+                        const int t = first_cell(tt[q], cells);
+                        if (cells > 0) S.cg_z[t] = __uint_as_float(fixed[0]);
+                    }
                     post(tt[q], z4, team.base | (pub + 1));
                 } else {
 #pragma unroll
@@ -554,12 +627,12 @@ __global__ void __launch_bounds__(256 * G, 1)
         {
             ok = exchange<3, NT>(team, nt, step, red, tsum, sums, bad, [&] { fetch(team.base | pub); },
                                  [&](const double (&tot)[3]) {
-                                     init_scalars(Ls, S, false, tot, n * n * n);
+                                     init_scalars(Ls, S, HEAT, tot, n * n * n);
                                      Ls.mean = (double)mean;
                                  });
         }
         // face fractions of the general tiles, zero where a face has no cell on one side (those terms drop out)
-        for (int q = g; q < nt; q += G) {
+        for (int q = g; !HEAT && q < nt; q += G) {
             if (tt[q].unit) continue;   // uniform in the group
             if (lt == 0) {
                 const int at = atomicAdd(&s_count[4], 1);
@@ -584,12 +657,6 @@ __global__ void __launch_bounds__(256 * G, 1)
             }
         }
         __syncthreads();
-        // the first of a tile's four cells, and which of them the domain has
-        auto first_cell = [&](const BrickTile& T, int& cells) {
-            const int j = T.j0 + row, k = T.k0 + lane;
-            cells = j < n && k < n ? min(4, n - T.i0) : 0;
-            return (T.i0 * n + j) * n + k;
-        };
         bool live = ok && Ls.live;
         int kit = 0;
         float beta = 0.0f;
@@ -608,9 +675,9 @@ __global__ void __launch_bounds__(256 * G, 1)
                     d[3] = dtab[c - (T.i0 + 4 == n)];
                 } else {
                     const bool in = j < n && k < n;
-                    const float* from = S.pdiag + (T.i0 * n + j) * n + k;
+                    const float* from = Dg + (T.i0 * n + j) * n + k;
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) d[m] = in && T.i0 + m < n ? from[m * n * n] : 0.0f;
+                    for (int m = 0; m < 4; ++m) d[m] = in && T.i0 + m < n ? from[m * nn] : 0.0f;
                 }
             }
         };
@@ -621,17 +688,17 @@ __global__ void __launch_bounds__(256 * G, 1)
             // p = z + beta p: the halo's copies and the block's own cells (the first p is z, placed by the set-up)
             take(team.base | (pub & 0x3ffu), [&](float& pb, float z) { pb = kit == 1 ? z : __fadd_rn(z, __fmul_rn(beta, pb)); });
             if (kit > 1) {
-#pragma unroll (kWide ? 3 : QR)
+#pragma unroll QR
                 for (int turn = 0; turn < turns; ++turn) {
                     const int s = kWide ? 0 : turn, q = G * turn + g;
                     if (q >= nt) continue;
                     float d[4], rv[4];
                     diag(tt[q], s, d);
                     float* core = sm + q * 1024 + lt;
-                    int cells;
-                    const int t = first_cell(tt[q], cells);
+                    int cells = 0;
+                    const int t = kWide ? first_cell(tt[q], cells) : 0;
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) rv[m] = !kWide ? r[s * 4 + m] : m < cells ? S.cg_r[t + m * n * n] : 0.0f;
+                    for (int m = 0; m < 4; ++m) rv[m] = !kWide ? r[s * 4 + m] : m < cells ? S.cg_r[t + m * nn] : 0.0f;
 #pragma unroll
                     for (int m = 0; m < 4; ++m) {
                         const float pv = __fadd_rn(__fmul_rn(d[m], rv[m]), __fmul_rn(beta, kKeepX ? pr[s * 4 + m] : core[m * 256]));
@@ -659,7 +726,35 @@ __global__ void __launch_bounds__(256 * G, 1)
 #pragma unroll
                 for (int m = 0; m < 4; ++m) p[m + 1] = kKeepX ? pr[s * 4 + m] : sm[core + m * 256];
                 float a[4];
-                if (T.unit) {
+                if constexpr (HEAT) {
+                    // heat.py:94-105: identity rows on fixed cells.  The solve takes an iteration or two, so the diffusivities
+                    // come from the lattices
+                    const int j = T.j0 + row, k = T.k0 + lane;
+                    if (kWide) {
+                        int cells;
+                        const int t = first_cell(T, cells);
+                        fixed[0] = cells > 0 ? __float_as_uint(S.cg_z[t]) : 0u;
+                    }
+#pragma unroll
+                    for (int m0 = 0; m0 < 4; m0 += 2) {
+                        float fx[3], fy[4], fz[4];
+                        coefficients(T.i0 + m0, j, k, fx, fy, fz);
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const int m = m0 + e;
+                            const unsigned mask = fixed[s] >> (8 * m);
+                            const float pc = p[m + 1];
+                            float acc = term(fx[e], mask & 1, pc, p[m]);
+                            acc = __fadd_rn(acc, term(fx[e + 1], mask & 2, pc, p[m + 2]));
+                            acc = __fadd_rn(acc, term(fy[e], mask & 4, pc, lo_j[m * 256]));
+                            acc = __fadd_rn(acc, term(fy[2 + e], mask & 8, pc, hi_j[m * 256]));
+                            acc = __fadd_rn(acc, term(fz[e], mask & 16, pc, lo_k[m * 256]));
+                            acc = __fadd_rn(acc, term(fz[2 + e], mask & 32, pc, hi_k[m * 256]));
+                            a[m] = mask & 64 ? pc : __fadd_rn(pc, __fmul_rn(c_dt, acc));
+                        }
+                        asm volatile("" ::: "memory");
+                    }
+                } else if (T.unit) {
 #pragma unroll
                     for (int m = 0; m < 4; ++m) {
                         const float pc = p[m + 1];
@@ -684,33 +779,27 @@ __global__ void __launch_bounds__(256 * G, 1)
                         a[m] = __fadd_rn(acc, __fmul_rn(fz[m * 264 + 1], __fsub_rn(pc, hi_k[m * 256])));
                     }
                 } else {
-                    // no box left: the fractions from the lattices, all requested before the first is used
-                    const int i0 = T.i0, j = T.j0 + row, k = T.k0 + lane;
-                    const bool in = j < n && k < n;
-                    float fx[5], fy[8], fz[8];
+                    // no box left: the fractions from the lattices
+                    const int j = T.j0 + row, k = T.k0 + lane;
 #pragma unroll
-                    for (int m = 0; m < 5; ++m)
-                        fx[m] = in && i0 + m > 0 && i0 + m < n ? __ldg(S.ax + uidx_(n, i0 + m, j, k)) : 0.0f;
+                    for (int m0 = 0; m0 < 4; m0 += 2) {
+                        float fx[3], fy[4], fz[4];
+                        coefficients(T.i0 + m0, j, k, fx, fy, fz);
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        const bool im = in && i0 + m < n;
-                        fy[m] = im && j > 0 ? __ldg(S.ay + vidx_(n, i0 + m, j, k)) : 0.0f;
-                        fy[4 + m] = im && j < n - 1 ? __ldg(S.ay + vidx_(n, i0 + m, j + 1, k)) : 0.0f;
-                        fz[m] = im && k > 0 ? __ldg(S.az + widx_(n, i0 + m, j, k)) : 0.0f;
-                        fz[4 + m] = im && k < n - 1 ? __ldg(S.az + widx_(n, i0 + m, j, k + 1)) : 0.0f;
-                    }
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        const float pc = p[m + 1];
-                        float acc = __fmul_rn(fx[m], __fsub_rn(pc, p[m]));
-                        acc = __fadd_rn(acc, __fmul_rn(fx[m + 1], __fsub_rn(pc, p[m + 2])));
-                        acc = __fadd_rn(acc, __fmul_rn(fy[m], __fsub_rn(pc, lo_j[m * 256])));
-                        acc = __fadd_rn(acc, __fmul_rn(fy[4 + m], __fsub_rn(pc, hi_j[m * 256])));
-                        acc = __fadd_rn(acc, __fmul_rn(fz[m], __fsub_rn(pc, lo_k[m * 256])));
-                        a[m] = __fadd_rn(acc, __fmul_rn(fz[4 + m], __fsub_rn(pc, hi_k[m * 256])));
+                        for (int e = 0; e < 2; ++e) {
+                            const int m = m0 + e;
+                            const float pc = p[m + 1];
+                            float acc = __fmul_rn(fx[e], __fsub_rn(pc, p[m]));
+                            acc = __fadd_rn(acc, __fmul_rn(fx[e + 1], __fsub_rn(pc, p[m + 2])));
+                            acc = __fadd_rn(acc, __fmul_rn(fy[e], __fsub_rn(pc, lo_j[m * 256])));
+                            acc = __fadd_rn(acc, __fmul_rn(fy[2 + e], __fsub_rn(pc, hi_j[m * 256])));
+                            acc = __fadd_rn(acc, __fmul_rn(fz[e], __fsub_rn(pc, lo_k[m * 256])));
+                            a[m] = __fadd_rn(acc, __fmul_rn(fz[2 + e], __fsub_rn(pc, hi_k[m * 256])));
+                        }
+                        asm volatile("" ::: "memory");
                     }
                 }
-                div_rn4(a, hhd);
+                if (!HEAT) div_rn4(a, hhd);
 #pragma unroll
                 for (int m = 0; m < 4; ++m) {
                     ap[s * 4 + m] = a[m];
@@ -721,7 +810,7 @@ __global__ void __launch_bounds__(256 * G, 1)
                     const int t = first_cell(T, cells);
 #pragma unroll
                     for (int m = 0; m < 4; ++m)
-                        if (m < cells) S.cg_Ap[t + m * n * n] = a[m];
+                        if (m < cells) S.cg_Ap[t + m * nn] = a[m];
                     stash(q, pAp);
                 }
             }
@@ -746,21 +835,21 @@ __global__ void __launch_bounds__(256 * G, 1)
                 float* x = sm + X + q * 1024 + lt;
                 if constexpr (kWide) {
                     int cells;
-                    const int t = first_cell(tt[q], cells), nn = n * n;
+                    const int t = first_cell(tt[q], cells);
                     float xv[4];
 #pragma unroll
                     for (int m = 0; m < 4; ++m) {
                         const bool in = m < cells;
                         r[m] = in ? S.cg_r[t + m * nn] : 0.0f;
                         ap[m] = in ? S.cg_Ap[t + m * nn] : 0.0f;
-                        xv[m] = in ? S.p[t + m * nn] : 0.0f;
+                        xv[m] = in ? xg[t + m * nn] : 0.0f;
                     }
 #pragma unroll
                     for (int m = 0; m < 4; ++m) {
                         r[m] = __fsub_rn(r[m], __fmul_rn(alpha, ap[m]));
                         if (m < cells) {
                             S.cg_r[t + m * nn] = r[m];
-                            S.p[t + m * nn] = __fadd_rn(xv[m], __fmul_rn(alpha, core[m * 256]));
+                            xg[t + m * nn] = __fadd_rn(xv[m], __fmul_rn(alpha, core[m * 256]));
                         }
                     }
                 }
@@ -792,15 +881,28 @@ __global__ void __launch_bounds__(256 * G, 1)
                                          Ls.iters = kit;
                                          if (!finite) Ls.status |= HF_SCENE_NONFINITE;
                                          Ls.live = above && finite && kit < Ls.maxit;
-                                         if (!Ls.live && above && finite) Ls.status |= HF_SCENE_PRESSURE_MAXITER;
+                                         if (!Ls.live && above && finite) Ls.status |= HEAT ? HF_SCENE_HEAT_MAXITER : HF_SCENE_PRESSURE_MAXITER;
                                      });
                 if (!ok) break;
                 beta = Ls.beta;
                 live = Ls.live;
             }
         }
-        // ------------------------------------------------------------- x back, projection of the faces (grid.py:140-153)
-        if (ok) {
+        // ------------------------------------------------------------- heat: x back
+        if (HEAT && !kWide && ok) {
+#pragma unroll QR
+            for (int turn = 0; turn < turns; ++turn) {
+                const int q = G * turn + g;
+                if (q >= nt) continue;
+                int cells;
+                const int t = first_cell(tt[q], cells);
+#pragma unroll
+                for (int m = 0; m < 4; ++m)
+                    if (m < cells) xg[t + m * nn] = kKeepX ? xr[turn * 4 + m] : sm[X + q * 1024 + m * 256 + lt];
+            }
+        }
+        // ------------------------------------------------------------- pressure: x back, projection (grid.py:140-153)
+        if (!HEAT && ok) {
             ++pub;
 #pragma unroll QR
             for (int turn = 0; turn < turns; ++turn) {
@@ -813,7 +915,7 @@ __global__ void __launch_bounds__(256 * G, 1)
                 for (int m = 0; m < 4; ++m) {
                     float& x = sm[X + q * 1024 + m * 256 + lt];
                     if (kKeepX) x = xr[s * 4 + m];
-                    if (kWide) x = m < cells ? S.p[t + m * n * n] : 0.0f;
+                    if (kWide) x = m < cells ? S.p[t + m * nn] : 0.0f;
                     x4[m] = x;
                 }
                 post(tt[q], x4, team.base | (pub & 0x3ffu));
@@ -822,46 +924,60 @@ __global__ void __launch_bounds__(256 * G, 1)
             if (warp >= kPollWarps) fetch(team.base | (pub & 0x3ffu));
             take(team.base | (pub & 0x3ffu), [&](float& pb, float v) { pb = v; });
             ok = !__syncthreads_or(bad);
-            if (bl.jobs > 1 && threadIdx.x == 0) {
-                asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ws.arrive + job) : "memory");
-                left = job;
-                left_nb = J.z;
-            }
         }
-        if (ok) {
+        if (!HEAT && ok) {
             float *u = S.u[par ^ 1], *v = S.v[par ^ 1], *w = S.w[par ^ 1];
             const float dtr = (float)(dt_d / S.rho);
+            const DivBy hd = div_by(h);
             for (int q = g; q < nt; q += G) {
                 const BrickTile& T = tt[q];
-                const TileItem it{0, T.i0, T.j0, T.k0};
                 auto at = [&](int o) { return o < X ? o + X : o; };   // the x of another tile of the block, or the halo
-                const int core = X + q * 1024 + lt;
+                const int core = X + q * 1024 + lt, j = T.j0 + row, k = T.k0 + lane;
                 const float* lo_j = sm + (row == 0 ? at(T.nb[2]) + lane : core - 32);
                 const float* lo_k = sm + (lane == 0 ? at(T.nb[4]) + row * 32 : core - 1);
-                float below = sm[at(T.nb[0]) + lt];
+                int cells;
+                const int t = first_cell(T, cells), fv = vidx_(n, T.i0, j, k), fw = widx_(n, T.i0, j, k);
+                // the tile's faces are requested together
+                float x[5], du[4], dv[4], dw[4], uo[4], vo[4], wo[4];
 #pragma unroll
                 for (int m = 0; m < 4; ++m) {
-                    const Cell cl = tile_cell(it, n, lt, m);
-                    const float pc = sm[core + m * 256];
-                    if (cl.ok) {
-                        if (!kWide) S.p[cl.t] = pc;
-                        const int i = cl.i, j = cl.j, k = cl.k;
-                        int f = uidx_(n, i, j, k);
-                        u[f] = i == 0 ? 0.0f : __fsub_rn(u[f], __fdiv_rn(__fmul_rn(dtr, __fsub_rn(pc, below)), h));
-                        f = vidx_(n, i, j, k);
-                        v[f] = j == 0 ? 0.0f : __fsub_rn(v[f], __fdiv_rn(__fmul_rn(dtr, __fsub_rn(pc, lo_j[m * 256])), h));
-                        f = widx_(n, i, j, k);
-                        w[f] = k == 0 ? 0.0f : __fsub_rn(w[f], __fdiv_rn(__fmul_rn(dtr, __fsub_rn(pc, lo_k[m * 256])), h));
-                        if (i == n - 1) u[uidx_(n, n, j, k)] = 0.0f;
-                        if (j == n - 1) v[vidx_(n, i, n, k)] = 0.0f;
-                        if (k == n - 1) w[widx_(n, i, j, n)] = 0.0f;
-                    }
-                    below = pc;
+                    const bool in = m < cells;
+                    uo[m] = in ? u[t + m * nn] : 0.0f;
+                    vo[m] = in ? v[fv + m * (nn + n)] : 0.0f;
+                    wo[m] = in ? w[fw + m * (nn + n)] : 0.0f;
+                }
+                x[0] = sm[at(T.nb[0]) + lt];
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    x[m + 1] = sm[core + m * 256];
+                    du[m] = __fmul_rn(dtr, __fsub_rn(x[m + 1], x[m]));
+                    dv[m] = __fmul_rn(dtr, __fsub_rn(x[m + 1], lo_j[m * 256]));
+                    dw[m] = __fmul_rn(dtr, __fsub_rn(x[m + 1], lo_k[m * 256]));
+                }
+                div_rn4(du, hd);
+                div_rn4(dv, hd);
+                div_rn4(dw, hd);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    if (m >= cells) continue;
+                    const int i = T.i0 + m;
+                    if (!kWide) S.p[t + m * nn] = x[m + 1];
+                    u[t + m * nn] = i == 0 ? 0.0f : __fsub_rn(uo[m], du[m]);
+                    v[fv + m * (nn + n)] = j == 0 ? 0.0f : __fsub_rn(vo[m], dv[m]);
+                    w[fw + m * (nn + n)] = k == 0 ? 0.0f : __fsub_rn(wo[m], dw[m]);
+                    if (i == n - 1) u[uidx_(n, n, j, k)] = 0.0f;
+                    if (j == n - 1) v[vidx_(n, i, n, k)] = 0.0f;
+                    if (k == n - 1) w[widx_(n, i, j, n)] = 0.0f;
                 }
             }
         }
         __syncthreads();
-        if (leader && threadIdx.x == 0) write_stats(S, Ls, false, !ok, par);
+        if (bl.jobs > 1 && threadIdx.x == 0) {
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ws.arrive + job) : "memory");
+            left = job;
+            left_nb = J.z;
+        }
+        if (leader && threadIdx.x == 0) write_stats(S, Ls, HEAT, !ok, par);
         __syncthreads();
     }
     // the last block to leave prepares the next launch: another launch number, no error, no arrivals
@@ -878,16 +994,21 @@ __global__ void __launch_bounds__(256 * G, 1)
     }
 }
 
-const void* brick_kernel(const BrickLaunch& bl, int* threads) {
-    // the small variants keep every tile's fractions in a box (launch_brick passes fewer boxes where they do not fit)
-    const int tiles = bl.boxes < bl.tiles && bl.tiles <= kBrickMaxTiles ? kBrickMaxTiles : bl.tiles;
+template <bool HEAT>
+static const void* pick(int tiles) {
+    if (tiles <= 2) return (const void*)k_brick<2, 1, HEAT>;
+    if (tiles <= 4) return (const void*)k_brick<4, 1, HEAT>;
+    if (tiles <= 6) return (const void*)k_brick<3, 2, HEAT>;
+    if (tiles <= 9) return (const void*)k_brick<3, 3, HEAT>;
+    if (tiles <= kBrickMaxTiles) return (const void*)k_brick<3, 5, HEAT>;
+    return (const void*)k_brick<3, 0, HEAT>;
+}
+
+const void* brick_kernel(const BrickLaunch& bl, bool heat, int* threads) {
+    // the small pressure variants keep every tile's fractions in a box (launch_brick passes fewer where they do not fit)
+    const int tiles = !heat && bl.boxes < bl.tiles && bl.tiles <= kBrickMaxTiles ? kBrickMaxTiles : bl.tiles;
     *threads = tiles <= 2 ? 512 : tiles <= 4 ? 1024 : 768;
-    if (tiles <= 2) return (const void*)k_brick<2, 1>;
-    if (tiles <= 4) return (const void*)k_brick<4, 1>;
-    if (tiles <= 6) return (const void*)k_brick<3, 2>;
-    if (tiles <= 9) return (const void*)k_brick<3, 3>;
-    if (tiles <= kBrickMaxTiles) return (const void*)k_brick<3, 5>;
-    return (const void*)k_brick<3, 0>;
+    return heat ? pick<true>(tiles) : pick<false>(tiles);
 }
 
 size_t brick_smem(const BrickLaunch& bl) {

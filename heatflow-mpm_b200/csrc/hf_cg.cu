@@ -19,16 +19,12 @@
 // Two grid barriers per iteration: the search direction p_k = z + beta p_{k-1} is not a separate phase -- every block
 // recomputes it at the stencil points it reads from z and the previous p (double-buffered), so it costs no barrier.
 //
-// Variants:
-//   k_pcg       streaming: vectors in global memory, any number of scenes (batched and served plans).  The scenes come
+// Variants (the on-chip solves of hf_brick.cu take the plans whose scenes fit there; these take the rest):
+//   k_pcg       streaming: vectors in global memory, any number of scenes.  The scenes come
 //               in L2-sized groups solved by the lanes of the grid; for the pressure system with every scene at
 //               n % 4 == 0 each tile's stencil boxes and CG vectors are staged by TMA from per-scene descriptors,
 //               double-buffered per block.  Optional outer defect correction (fp64 true residual, restart).
-//   k_pcg_res   register-resident, one scene: every thread keeps x, r, z, p, D and Ap of its cells in registers for
-//               the whole solve; only p and z are published (neighbouring blocks read them).
-//   k_pcg_tma   register-resident pressure solve of one scene with n % 4 == 0: the stencil inputs of each tile -- z
-//               and the previous p with a one-cell halo, and the face fractions -- are staged into shared memory by
-//               TMA (cp.async.bulk.tensor) instead of gathered; x, r and D stay in registers.
+//   k_pcg_one   pressure solve of one scene with n % 4 == 0 with one grid barrier per iteration (see there).
 #include <cuda.h>
 
 #include "hf_cg.cuh"
@@ -336,44 +332,10 @@ struct Vec {
     __device__ __forceinline__ float operator()(int t) const { return a[t]; }
 };
 
-// grid.py:94-115 k_laplacian accumulation: sum over the six faces of alpha_f (x_c - x_nb), domain faces skipped
-template <class X>
-__device__ __forceinline__ float lap_acc(const hf_scene& S, const X& x, float xc, int t, int i, int j, int k) {
-    const int n = S.n, nn = n * n;
-    float acc = 0.0f;
-    if (i > 0) acc = __fadd_rn(acc, __fmul_rn(__ldg(S.ax + uidx_(n, i, j, k)), __fsub_rn(xc, x(t - nn))));
-    if (i < n - 1) acc = __fadd_rn(acc, __fmul_rn(__ldg(S.ax + uidx_(n, i + 1, j, k)), __fsub_rn(xc, x(t + nn))));
-    if (j > 0) acc = __fadd_rn(acc, __fmul_rn(__ldg(S.ay + vidx_(n, i, j, k)), __fsub_rn(xc, x(t - n))));
-    if (j < n - 1) acc = __fadd_rn(acc, __fmul_rn(__ldg(S.ay + vidx_(n, i, j + 1, k)), __fsub_rn(xc, x(t + n))));
-    if (k > 0) acc = __fadd_rn(acc, __fmul_rn(__ldg(S.az + widx_(n, i, j, k)), __fsub_rn(xc, x(t - 1))));
-    if (k < n - 1) acc = __fadd_rn(acc, __fmul_rn(__ldg(S.az + widx_(n, i, j, k + 1)), __fsub_rn(xc, x(t + 1))));
-    return acc;
-}
-
-// heat.py:55-91 neighbour_terms with use_fixed = 0; kappa_f from the precomputed face diffusivities
-template <class X>
-__device__ __forceinline__ float heat_nt(const hf_scene& S, const X& x, float xc, int t, int i, int j, int k) {
-    const int n = S.n, nn = n * n;
-    const uint8_t* __restrict__ fl = S.cell_flags;
-    float acc = 0.0f;
-    const int nbr[6] = {t - nn, t + nn, t - n, t + n, t - 1, t + 1};
-    const bool in[6] = {i > 0, i < n - 1, j > 0, j < n - 1, k > 0, k < n - 1};
-    const int fidx[6] = {uidx_(n, i, j, k), uidx_(n, i + 1, j, k), vidx_(n, i, j, k), vidx_(n, i, j + 1, k),
-                         widx_(n, i, j, k), widx_(n, i, j, k + 1)};
-    const float* __restrict__ hk[3] = {S.hkx, S.hky, S.hkz};
-#pragma unroll
-    for (int s = 0; s < 6; ++s) {
-        if (!in[s]) continue;
-        const int nb = nbr[s];
-        const float kf = __ldg(hk[s >> 1] + fidx[s]);
-        acc = __fadd_rn(acc, (__ldg(fl + nb) & 1) ? __fmul_rn(kf, xc) : __fmul_rn(kf, __fsub_rn(xc, x(nb))));
-    }
-    return acc;
-}
-
-// The same two sums with every load hoisted, for the streaming kernel, where each thread's loads should all be in
-// flight at once.  Every load is in bounds (a missing neighbour reads the cell itself, face fractions exist on all n+1 layers), so all
-// of them can be in flight at once; the terms of domain faces are then left out of the sum, in the reference's order.
+// grid.py:94-115 k_laplacian accumulation, the sum over the six faces of alpha_f (x_c - x_nb) with domain faces skipped,
+// every load hoisted: each is in bounds (a missing neighbour reads the cell itself, face fractions exist on all n+1
+// layers), so all of a thread's loads are in flight at once; the terms of domain faces are then left out of the sum, in
+// the reference's order.
 template <class X>
 __device__ __forceinline__ float lap_acc_hoisted(const hf_scene& S, const X& x, float xc, int t, int i, int j, int k) {
     const int n = S.n, nn = n * n;
@@ -394,7 +356,7 @@ __device__ __forceinline__ float lap_acc_hoisted(const hf_scene& S, const X& x, 
 }
 
 // heat.py:55-91 neighbour_terms with use_fixed = 0; kappa_f from the precomputed face diffusivities (loads hoisted
-// and kept in bounds as in lap_acc)
+// and kept in bounds as in lap_acc_hoisted)
 template <class X>
 __device__ __forceinline__ float heat_nt_hoisted(const hf_scene& S, const X& x, float xc, int t, int i, int j, int k) {
     const int n = S.n, nn = n * n;
@@ -545,11 +507,6 @@ __device__ double true_residual_heat(const hf_scene& S, const float* __restrict_
 // Out-of-range elements are zero-filled by the copy engine and never used (domain faces are skipped).
 constexpr int kBZ = 40 * 10 * 6, kBX = 32 * 8 * 5, kBY = 32 * 9 * 4, kBW = 36 * 8 * 4;
 constexpr int kSlotFloats = 2 * kBZ + kBX + kBY + kBW;   // 8384 floats = 33,536 bytes (a multiple of 128)
-// Heat system: the same z / p boxes; face diffusivities x (face lattice), y (face lattice: rows j0..j0+8 of (n, n+1, n))
-// and z (cell-layout copy) in the face-fraction places; the cell flags (bytes) k in [k0-16, k0+48), j in [j0-1, j0+9),
-// i in [i0-1, i0+5) -- 16-byte aligned k origin; the owner's and the neighbours' fixed bits.
-constexpr int kBF = 64 * 10 * 6;                                   // bytes
-constexpr int kHeatSlotFloats = kSlotFloats + kBF / 4;             // 9344 floats = 37,376 bytes (a multiple of 128)
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -1095,719 +1052,6 @@ __global__ void __launch_bounds__(kThreads) k_pcg(const hf_scene* __restrict__ s
     }
 }
 
-// ======================================================================================= register-resident
-// Block = `groups` x 256 threads; group g owns tiles c0 + g + groups*q (q < MAXC) of the block's contiguous range.
-template <bool HEAT, int MAXC, bool TMA>
-__global__ void __launch_bounds__(MAXC == 1 ? 1024 : (MAXC == 2 ? 768 : 512), 1)
-    k_pcg_res(const hf_scene* __restrict__ scenes, const TileItem* __restrict__ tiles, int tile_lo, int tile_hi,
-              double dt_d, Workspace ws, const __grid_constant__ TileMaps maps) {
-    constexpr int CPT = 4 * MAXC;   // cells per thread
-    extern __shared__ __align__(128) float sm_raw[];
-    // TMA destinations must be 128-byte aligned: the launch adds 128 bytes of slack
-    float* sm_boxes = align128_shared(sm_raw);
-    __shared__ double red[kRedComps * 32];
-    __shared__ LocalScene Ls;
-    __shared__ __align__(8) unsigned long long mbar[4 * 3];
-    __shared__ TileItem my_s[4 * 3];
-    const int groups = blockDim.x >> 8, g = threadIdx.x >> 8, lt = threadIdx.x & 255;
-    const int c0 = tile_lo + (int)(((long long)(tile_hi - tile_lo) * blockIdx.x) / gridDim.x);
-    const int c1 = tile_lo + (int)(((long long)(tile_hi - tile_lo) * (blockIdx.x + 1)) / gridDim.x);
-    const int sidx = tiles[c0].scene;   // one scene per plan on this path
-    const hf_scene& S = scenes[sidx];
-    const int n = S.n, N = n * n * n;
-    const int par = S.state->parity;
-    unsigned* bar = ws.bar + (HEAT ? 0 : kMaxLanes);
-    unsigned epoch = 0;
-    const float dt = (float)dt_d;
-    const float h = (float)S.h, hh = __fmul_rn(h, h), c_dt = __fdiv_rn(dt, hh);
-    double* bufA = ws.partA;
-    double* bufB = ws.partB;
-    const int cb = ws.tile_begin[sidx], ce = ws.tile_begin[sidx + 1];
-    float* xg = HEAT ? S.T[par ^ 1] : S.p;
-    float* zg = S.cg_z;
-    // the group's tiles in shared memory (registers held through the solve make the stencil phases spill)
-    TileItem* const my = my_s + g * MAXC;
-    bool have[MAXC];
-#pragma unroll
-    for (int q = 0; q < MAXC; ++q) have[q] = c0 + g + groups * q < c1;
-    if (lt < MAXC) {
-        const int c = c0 + g + groups * lt;
-        my[lt] = tiles[c < c1 ? c : c0];
-    }
-    unsigned phase_bit = 0;
-    if (TMA && lt == 0) {
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) mbar_init(&mbar[g * MAXC + q], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-
-    float x[CPT], r[CPT], z[CPT], p[CPT], D[CPT], Ap[CPT];
-    // ------------------------------------------------------------------ prologue (values kept in registers)
-    float mean = 0.0f;
-    if (!HEAT) {
-        double mm[1];
-        const int comp[1] = {0};
-        scene_sums<1>(ws.mean_part, ws.chunk_begin[sidx], ws.chunk_begin[sidx + 1], comp, mm, red, 0);
-        mean = __double2float_rn(mm[0] / ((double)n * n * n));
-    }
-#pragma unroll
-    for (int q = 0; q < MAXC; ++q) {
-        double part[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const int s = q * 4 + m;
-            x[s] = r[s] = z[s] = p[s] = D[s] = Ap[s] = 0.0f;
-            const Cell cl = tile_cell(my[q], n, lt, m);
-            if (!have[q] || !cl.ok) continue;
-            float b, d, rr;
-            setup_cell<HEAT>(S, xg, mean, hh, c_dt, cl, b, d, rr);
-            x[s] = xg[cl.t];
-            D[s] = d;
-            r[s] = rr;
-            z[s] = __fmul_rn(d, rr);
-            zg[cl.t] = z[s];
-            part[0] += (double)b * (double)b;
-            part[1] += (double)rr * (double)rr;
-            part[2] += (double)rr * (double)z[s];
-        }
-        group_sum<3>(part, red);
-        const int c = c0 + g + groups * q;
-        if (lt == 0 && have[q]) {
-            bufB[c] = part[0];
-            bufB[1 * ws.tiles + c] = part[1];
-            bufB[2 * ws.tiles + c] = part[2];
-        }
-    }
-    // the face fractions of the tiles stay in shared memory for the whole solve
-    if (TMA && lt == 0) {
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) {
-            if (!have[q]) continue;
-            float* slot = sm_boxes + (size_t)(g * MAXC + q) * kSlotFloats;
-            unsigned long long* mb = &mbar[g * MAXC + q];
-            mbar_expect_tx(mb, (unsigned)((kBX + kBY + kBW) * sizeof(float)));
-            tma_load_3d(slot + 2 * kBZ, &maps.ax, my[q].k0, my[q].j0, my[q].i0, mb);
-            tma_load_3d(slot + 2 * kBZ + kBX, &maps.ayc, my[q].k0, my[q].j0, my[q].i0, mb);
-            tma_load_3d(slot + 2 * kBZ + kBX + kBY, &maps.azc, my[q].k0, my[q].j0, my[q].i0, mb);
-        }
-    }
-    if (TMA) {
-        bool ok = true;
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q)
-            if (have[q]) ok = mbar_wait(&mbar[g * MAXC + q], phase_bit) && ok;
-        if (!ok) atomicExch(ws.err, 1);
-        phase_bit ^= 1u;
-    }
-    if (!grid_barrier(bar, epoch, ws.err, gridDim.x)) goto finish;
-    {
-        double tot[3];
-        const int comp[3] = {0, 1, 2};
-        scene_sums<3>(bufB, cb, ce, comp, tot, red, ws.tiles);
-        if (threadIdx.x == 0) {
-            init_scalars(Ls, S, HEAT, tot, N);
-            Ls.mean = (double)mean;
-        }
-        __syncthreads();
-    }
-    // ------------------------------------------------------------------------------------------ iterations
-    for (int kit = 1; Ls.live; ++kit) {
-        // phase A: p_k, Ap = A p_k, p.Ap
-        const float beta = Ls.beta;
-        const bool first = kit == 1;
-        const float* pold = S.cg_p[(kit - 1) & 1];
-        float* pnew = S.cg_p[kit & 1];
-        if (TMA) {
-            // stage z and p_{k-1} (with halo) of every tile of the group, then form p_k in place over the z box
-            if (lt == 0) {
-                asm volatile("fence.proxy.async.global;" ::: "memory");
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-#pragma unroll
-                for (int q = 0; q < MAXC; ++q) {
-                    if (!have[q]) continue;
-                    float* slot = sm_boxes + (size_t)(g * MAXC + q) * kSlotFloats;
-                    unsigned long long* mb = &mbar[g * MAXC + q];
-                    mbar_expect_tx(mb, (unsigned)((first ? 1 : 2) * kBZ * sizeof(float)));
-                    tma_load_3d(slot, &maps.z, my[q].k0 - 4, my[q].j0 - 1, my[q].i0 - 1, mb);
-                    if (!first)
-                        tma_load_3d(slot + kBZ, ((kit - 1) & 1) ? &maps.p1 : &maps.p0, my[q].k0 - 4, my[q].j0 - 1,
-                                    my[q].i0 - 1, mb);
-                }
-            }
-            bool ok = true;
-#pragma unroll
-            for (int q = 0; q < MAXC; ++q)
-                if (have[q]) ok = mbar_wait(&mbar[g * MAXC + q], phase_bit) && ok;
-            if (!ok) atomicExch(ws.err, 1);
-            phase_bit ^= 1u;
-            if (!first) {
-#pragma unroll
-                for (int q = 0; q < MAXC; ++q) {
-                    if (!have[q]) continue;
-                    float* slot = sm_boxes + (size_t)(g * MAXC + q) * kSlotFloats;
-                    for (int e = lt; e < kBZ; e += 256) slot[e] = __fadd_rn(slot[e], __fmul_rn(beta, slot[kBZ + e]));
-                }
-            }
-            asm volatile("bar.sync %0, 256;" ::"r"(g + 1) : "memory");
-#pragma unroll
-            for (int q = 0; q < MAXC; ++q) {
-                const float* slot = sm_boxes + (size_t)(g * MAXC + q) * kSlotFloats;
-                const float* Pb = slot;
-                const float* axb = slot + 2 * kBZ;
-                const float* ayb = axb + kBX;
-                const float* azb = ayb + kBY;
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const int s = q * 4 + m;
-                    const Cell cl = tile_cell(my[q], n, lt, m);
-                    if (!have[q] || !cl.ok) continue;
-                    const float pc = first ? z[s] : __fadd_rn(z[s], __fmul_rn(beta, p[s]));
-                    const int bi = cl.i - my[q].i0, bj = cl.j - my[q].j0, bk = cl.k - my[q].k0;
-                    const int o = (bi + 1) * 400 + (bj + 1) * 40 + (bk + 4);
-                    float acc = 0.0f;
-                    if (cl.i > 0) acc = __fadd_rn(acc, __fmul_rn(axb[bi * 256 + bj * 32 + bk], __fsub_rn(pc, Pb[o - 400])));
-                    if (cl.i < n - 1)
-                        acc = __fadd_rn(acc, __fmul_rn(axb[(bi + 1) * 256 + bj * 32 + bk], __fsub_rn(pc, Pb[o + 400])));
-                    if (cl.j > 0) acc = __fadd_rn(acc, __fmul_rn(ayb[bi * 288 + bj * 32 + bk], __fsub_rn(pc, Pb[o - 40])));
-                    if (cl.j < n - 1)
-                        acc = __fadd_rn(acc, __fmul_rn(ayb[bi * 288 + (bj + 1) * 32 + bk], __fsub_rn(pc, Pb[o + 40])));
-                    if (cl.k > 0) acc = __fadd_rn(acc, __fmul_rn(azb[bi * 288 + bj * 36 + bk], __fsub_rn(pc, Pb[o - 1])));
-                    if (cl.k < n - 1)
-                        acc = __fadd_rn(acc, __fmul_rn(azb[bi * 288 + bj * 36 + bk + 1], __fsub_rn(pc, Pb[o + 1])));
-                    Ap[s] = __fdiv_rn(acc, hh);
-                    p[s] = pc;
-                }
-            }
-        } else {
-            const Dir P{zg, pold, beta, first};
-#pragma unroll
-            for (int q = 0; q < MAXC; ++q) {
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const int s = q * 4 + m;
-                    const Cell cl = tile_cell(my[q], n, lt, m);
-                    if (!have[q] || !cl.ok) continue;
-                    const float pc = first ? z[s] : __fadd_rn(z[s], __fmul_rn(beta, p[s]));
-                    if (HEAT) {
-                        Ap[s] = (__ldg(S.cell_flags + cl.t) & 1)
-                                    ? pc
-                                    : __fadd_rn(pc, __fmul_rn(c_dt, heat_nt(S, P, pc, cl.t, cl.i, cl.j, cl.k)));
-                    } else {
-                        Ap[s] = __fdiv_rn(lap_acc(S, P, pc, cl.t, cl.i, cl.j, cl.k), hh);
-                    }
-                    p[s] = pc;
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) {
-            double part[1] = {0.0};
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const int s = q * 4 + m;
-                const Cell cl = tile_cell(my[q], n, lt, m);
-                if (!have[q] || !cl.ok) continue;
-                pnew[cl.t] = p[s];
-                part[0] += (double)p[s] * (double)Ap[s];
-            }
-            group_sum<1>(part, red);
-            const int c = c0 + g + groups * q;
-            if (lt == 0 && have[q]) bufA[c] = part[0];
-        }
-        if (!grid_barrier(bar, epoch, ws.err, gridDim.x)) goto finish;
-        {
-            double tot[1];
-            const int comp[1] = {0};
-            scene_sums<1>(bufA, cb, ce, comp, tot, red, ws.tiles);
-            if (threadIdx.x == 0) {
-                Ls.pAp = tot[0];
-                Ls.alpha = __double2float_rn(Ls.rz / tot[0]);
-            }
-            __syncthreads();
-        }
-        // phase B: x += alpha p, r -= alpha Ap, z = D r (registers), publish z, r.r and r.z
-        const float alpha = Ls.alpha;
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) {
-            double part[2] = {0.0, 0.0};
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const int s = q * 4 + m;
-                const Cell cl = tile_cell(my[q], n, lt, m);
-                if (!have[q] || !cl.ok) continue;
-                x[s] = __fadd_rn(x[s], __fmul_rn(alpha, p[s]));
-                r[s] = __fsub_rn(r[s], __fmul_rn(alpha, Ap[s]));
-                z[s] = __fmul_rn(D[s], r[s]);
-                zg[cl.t] = z[s];
-                part[0] += (double)r[s] * (double)r[s];
-                part[1] += (double)r[s] * (double)z[s];
-            }
-            group_sum<2>(part, red);
-            const int c = c0 + g + groups * q;
-            if (lt == 0 && have[q]) {
-                bufB[1 * ws.tiles + c] = part[0];
-                bufB[2 * ws.tiles + c] = part[1];
-            }
-        }
-        if (!grid_barrier(bar, epoch, ws.err, gridDim.x)) goto finish;
-        {
-            double tot[2];
-            const int comp[2] = {1, 2};
-            scene_sums<2>(bufB, cb, ce, comp, tot, red, ws.tiles);
-            if (threadIdx.x == 0) update_scalars(Ls, HEAT, tot[0], tot[1], kit);
-            __syncthreads();
-        }
-    }
-    // ------------------------------------------------------------------ write the solution back
-#pragma unroll
-    for (int q = 0; q < MAXC; ++q) {
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const Cell cl = tile_cell(my[q], n, lt, m);
-            if (have[q] && cl.ok) xg[cl.t] = x[q * 4 + m];
-        }
-    }
-    if (!HEAT) {
-        // grid.py:140-153: the projection reads p at neighbour cells owned by other blocks
-        if (!grid_barrier(bar, epoch, ws.err, gridDim.x)) goto finish;
-        const float dtr = (float)(dt_d / S.rho);
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) {
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const Cell cl = tile_cell(my[q], n, lt, m);
-                if (have[q] && cl.ok)
-                    project_cell(S, S.u[par ^ 1], S.v[par ^ 1], S.w[par ^ 1], S.p, x[q * 4 + m], dtr, h, cl);
-            }
-        }
-    }
-finish:
-    if (TMA && *(volatile int*)ws.err) {
-        // leave no copy in flight: a timed-out wait is retried (bounded) before the block exits
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q)
-            if (have[q]) mbar_wait(&mbar[g * MAXC + q], phase_bit ^ 1u);
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) write_stats(S, Ls, HEAT, *(volatile int*)ws.err != 0, par);
-}
-
-// ============================================================================= resident pressure CG with TMA staging
-// Same mapping, arithmetic and reduction trees as k_pcg / k_pcg_res, with less state per thread: the search direction
-// of the own cells is read from the staged box (its centre), A p is parked in the p_{k-1} box (dead once p_k is
-// formed), so a thread keeps only x, r and D of its cells in registers.  One group reduction per phase covers all the
-// thread's tiles.
-// Set-up of one heat cell from the staged boxes (x0 with a one-cell halo at B, then the face-diffusivity boxes and the
-// flag byte box at F): setup_cell<true>'s operations in its order on the same values (heat.py:198-203 with k_heat_diag
-// and neighbour_terms, use_fixed = 0).  Box offsets as in the iterations' stencil.
-__device__ __forceinline__ void heat_setup_box(const float* __restrict__ B, const float* __restrict__ F, float b, float c_dt,
-                                               const Cell& cl, int n, int bi, int bj, int bk, float& bo, float& d,
-                                               float& r, float& xo) {
-    const float* axb = F;
-    const float* ayb = axb + kBX;
-    const float* azb = ayb + kBY;
-    const unsigned char* flb = reinterpret_cast<const unsigned char*>(azb + kBW);
-    const int o = (bi + 1) * 400 + (bj + 1) * 40 + (bk + 4);
-    const int of = (bi + 1) * 640 + (bj + 1) * 64 + (bk + 16);
-    const float xc = B[o];
-    bo = b;
-    xo = xc;
-    if (flb[of] & 1) {
-        d = 1.0f;
-        r = __fsub_rn(b, xc);
-        return;
-    }
-    const bool in[6] = {cl.i > 0, cl.i < n - 1, cl.j > 0, cl.j < n - 1, cl.k > 0, cl.k < n - 1};
-    const float kf[6] = {axb[bi * 256 + bj * 32 + bk], axb[(bi + 1) * 256 + bj * 32 + bk], ayb[bi * 288 + bj * 32 + bk],
-                         ayb[bi * 288 + (bj + 1) * 32 + bk], azb[bi * 288 + bj * 36 + bk], azb[bi * 288 + bj * 36 + bk + 1]};
-    const int step[6] = {-400, 400, -40, 40, -1, 1}, fstep[6] = {-640, 640, -64, 64, -1, 1};
-    float sd = 0.0f, nt = 0.0f;
-#pragma unroll
-    for (int s = 0; s < 6; ++s)
-        if (in[s]) sd = __fadd_rn(sd, kf[s]);
-#pragma unroll
-    for (int s = 0; s < 6; ++s) {
-        if (!in[s]) continue;
-        nt = __fadd_rn(nt, (flb[of + fstep[s]] & 1) ? __fmul_rn(kf[s], xc) : __fmul_rn(kf[s], __fsub_rn(xc, B[o + step[s]])));
-    }
-    d = __fdiv_rn(1.0f, __fadd_rn(1.0f, __fmul_rn(c_dt, sd)));
-    r = __fsub_rn(b, __fadd_rn(xc, __fmul_rn(c_dt, nt)));
-}
-
-template <bool HEAT, int MAXC>
-__global__ void __launch_bounds__(MAXC == 1 ? 1024 : (MAXC == 2 ? 768 : 512), 1)
-    k_pcg_tma(const hf_scene* __restrict__ scenes, const TileItem* __restrict__ tiles, int tile_lo, int tile_hi,
-              double dt_d, Workspace ws, const __grid_constant__ TileMaps maps) {
-    constexpr int CPT = 4 * MAXC;
-    constexpr int SLOT = HEAT ? kHeatSlotFloats : kSlotFloats;
-    extern __shared__ __align__(128) float sm_raw[];
-    float* sm_boxes = align128_shared(sm_raw);
-    __shared__ double red[kRedComps * 32];
-    __shared__ LocalScene Ls;
-    __shared__ __align__(8) unsigned long long mbar[4 * 3];
-    __shared__ TileItem my_s[4 * 3];
-    const int groups = blockDim.x >> 8, g = threadIdx.x >> 8, lt = threadIdx.x & 255;
-    const int c0 = tile_lo + (int)(((long long)(tile_hi - tile_lo) * blockIdx.x) / gridDim.x);
-    const int c1 = tile_lo + (int)(((long long)(tile_hi - tile_lo) * (blockIdx.x + 1)) / gridDim.x);
-    const int sidx = tiles[c0].scene;
-    const hf_scene& S = scenes[sidx];
-    const int n = S.n, N = n * n * n;
-    const int par = S.state->parity;
-    unsigned* bar = ws.bar + (HEAT ? 0 : kMaxLanes);
-    unsigned epoch = 0;
-    const float h = (float)S.h, hh = __fmul_rn(h, h), c_dt = __fdiv_rn((float)dt_d, hh);
-    const DivBy hhd = div_by(hh);
-    double* bufA = ws.partA;
-    double* bufB = ws.partB;
-    const int cb = ws.tile_begin[sidx], ce = ws.tile_begin[sidx + 1];
-    float* xg = HEAT ? S.T[par ^ 1] : S.p;
-    float* zg = S.cg_z;
-    // the group's tiles in shared memory (registers held through the solve make the stencil phases spill)
-    TileItem* const my = my_s + g * MAXC;
-    bool have[MAXC];
-#pragma unroll
-    for (int q = 0; q < MAXC; ++q) have[q] = c0 + g + groups * q < c1;
-    if (lt < MAXC) {
-        const int c = c0 + g + groups * lt;
-        my[lt] = tiles[c < c1 ? c : c0];
-    }
-    unsigned phase_bit = 0;
-    // the z and p_{k-1} boxes of iteration kit, requested by thread lt == 0 of each group; the next iteration's are
-    // requested right after the barrier that ends phase B, before the scene sums, so the copy overlaps them
-    auto issue_boxes = [&](int kit) {
-        if (lt != 0) return;
-        asm volatile("fence.proxy.async.global;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) {
-            if (!have[q]) continue;
-            float* slot = sm_boxes + (size_t)(g * MAXC + q) * SLOT;
-            unsigned long long* mb = &mbar[g * MAXC + q];
-            mbar_expect_tx(mb, (unsigned)((kit == 1 ? 1 : 2) * kBZ * sizeof(float)));
-            tma_load_3d(slot, &maps.z, my[q].k0 - 4, my[q].j0 - 1, my[q].i0 - 1, mb);
-            if (kit != 1)
-                tma_load_3d(slot + kBZ, ((kit - 1) & 1) ? &maps.p1 : &maps.p0, my[q].k0 - 4, my[q].j0 - 1, my[q].i0 - 1,
-                            mb);
-        }
-    };
-    bool requested = false;   // the next iteration's boxes are in flight
-    if (lt == 0) {
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) mbar_init(&mbar[g * MAXC + q], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    float x[CPT], r[CPT], D[CPT];
-    // heat: x0 (the advected T, into the z slot), the face diffusivities and the cell flags with halo are staged by
-    // TMA before the set-up, which then reads them from shared memory; the coefficient boxes stay for the whole solve
-    if (HEAT) {
-        if (lt == 0) {
-            asm volatile("fence.proxy.async.global;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-#pragma unroll
-            for (int q = 0; q < MAXC; ++q) {
-                if (!have[q]) continue;
-                float* slot = sm_boxes + (size_t)(g * MAXC + q) * SLOT;
-                unsigned long long* mb = &mbar[g * MAXC + q];
-                mbar_expect_tx(mb, (unsigned)((kBZ + kBX + kBY + kBW) * sizeof(float) + kBF));
-                tma_load_3d(slot, (par ^ 1) ? &maps.t1 : &maps.t0, my[q].k0 - 4, my[q].j0 - 1, my[q].i0 - 1, mb);
-                tma_load_3d(slot + 2 * kBZ, &maps.hkx, my[q].k0, my[q].j0, my[q].i0, mb);
-                tma_load_3d(slot + 2 * kBZ + kBX, &maps.hky, my[q].k0, my[q].j0, my[q].i0, mb);
-                tma_load_3d(slot + 2 * kBZ + kBX + kBY, &maps.hkzc, my[q].k0, my[q].j0, my[q].i0, mb);
-                tma_load_3d(slot + 2 * kBZ + kBX + kBY + kBW, &maps.flags, my[q].k0 - 16, my[q].j0 - 1, my[q].i0 - 1, mb);
-            }
-        }
-        bool ok = true;
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q)
-            if (have[q]) ok = mbar_wait(&mbar[g * MAXC + q], phase_bit) && ok;
-        if (!ok) atomicExch(ws.err, 1);
-        phase_bit ^= 1u;
-    }
-    // ------------------------------------------------------------------------------------------ prologue
-    float mean = 0.0f;
-    if (!HEAT) {
-        double mm[1];
-        const int comp[1] = {0};
-        scene_sums<1>(ws.mean_part, ws.chunk_begin[sidx], ws.chunk_begin[sidx + 1], comp, mm, red, 0);
-        mean = __double2float_rn(mm[0] / ((double)n * n * n));
-    }
-    {
-        double part[3 * MAXC];
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) {
-            part[3 * q] = part[3 * q + 1] = part[3 * q + 2] = 0.0;
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const int s = q * 4 + m;
-                x[s] = r[s] = D[s] = 0.0f;
-                const Cell cl = tile_cell(my[q], n, lt, m);
-                if (!have[q] || !cl.ok) continue;
-                float b, d, rr, xc;
-                if (HEAT) {
-                    const float* slot = sm_boxes + (size_t)(g * MAXC + q) * SLOT;
-                    heat_setup_box(slot, slot + 2 * kBZ, S.hrhs[cl.t], c_dt, cl, n, m, lt >> 5, lt & 31, b, d, rr, xc);
-                } else {
-                    setup_cell<HEAT>(S, xg, mean, hh, c_dt, cl, b, d, rr);
-                    xc = xg[cl.t];
-                }
-                const float z = __fmul_rn(d, rr);
-                x[s] = xc;
-                D[s] = d;
-                r[s] = rr;
-                zg[cl.t] = z;
-                part[3 * q] += (double)b * (double)b;
-                part[3 * q + 1] += (double)rr * (double)rr;
-                part[3 * q + 2] += (double)rr * (double)z;
-            }
-        }
-        group_sum<3 * MAXC>(part, red);
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) {
-            const int c = c0 + g + groups * q;
-            if (lt == 0 && have[q]) {
-                bufB[c] = part[3 * q];
-                bufB[1 * ws.tiles + c] = part[3 * q + 1];
-                bufB[2 * ws.tiles + c] = part[3 * q + 2];
-            }
-        }
-    }
-    // the tiles' face fractions stay in shared memory for the whole solve (heat: staged before the set-up)
-    if (!HEAT && lt == 0) {
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) {
-            if (!have[q]) continue;
-            float* slot = sm_boxes + (size_t)(g * MAXC + q) * SLOT;
-            unsigned long long* mb = &mbar[g * MAXC + q];
-            mbar_expect_tx(mb, (unsigned)((kBX + kBY + kBW) * sizeof(float)));
-            tma_load_3d(slot + 2 * kBZ, &maps.ax, my[q].k0, my[q].j0, my[q].i0, mb);
-            tma_load_3d(slot + 2 * kBZ + kBX, &maps.ayc, my[q].k0, my[q].j0, my[q].i0, mb);
-            tma_load_3d(slot + 2 * kBZ + kBX + kBY, &maps.azc, my[q].k0, my[q].j0, my[q].i0, mb);
-        }
-    }
-    if (!HEAT) {
-        bool ok = true;
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q)
-            if (have[q]) ok = mbar_wait(&mbar[g * MAXC + q], phase_bit) && ok;
-        if (!ok) atomicExch(ws.err, 1);
-        phase_bit ^= 1u;
-    }
-    if (!grid_barrier(bar, epoch, ws.err, gridDim.x)) goto finish;
-    issue_boxes(1);
-    requested = true;
-    {
-        double tot[3];
-        const int comp[3] = {0, 1, 2};
-        scene_sums<3>(bufB, cb, ce, comp, tot, red, ws.tiles);
-        if (threadIdx.x == 0) {
-            init_scalars(Ls, S, HEAT, tot, N);
-            Ls.mean = (double)mean;
-        }
-        __syncthreads();
-    }
-    // ------------------------------------------------------------------------------------------ iterations
-    for (int kit = 1; Ls.live; ++kit) {
-        const float beta = Ls.beta;
-        const bool first = kit == 1;
-        float* pnew = S.cg_p[kit & 1];
-        // phase A: stage z and p_{k-1} with halo (requested after the previous barrier), form p_k in place, Ap from
-        // shared memory
-        if (!requested) issue_boxes(kit);
-        requested = false;
-        {
-            bool ok = true;
-#pragma unroll
-            for (int q = 0; q < MAXC; ++q)
-                if (have[q]) ok = mbar_wait(&mbar[g * MAXC + q], phase_bit) && ok;
-            if (!ok) atomicExch(ws.err, 1);
-            phase_bit ^= 1u;
-        }
-        if (!first) {
-#pragma unroll
-            for (int q = 0; q < MAXC; ++q) {
-                if (!have[q]) continue;
-                float* slot = sm_boxes + (size_t)(g * MAXC + q) * SLOT;
-                for (int e = lt; e < kBZ; e += 256) slot[e] = __fadd_rn(slot[e], __fmul_rn(beta, slot[kBZ + e]));
-            }
-        }
-        asm volatile("bar.sync %0, 256;" ::"r"(g + 1) : "memory");
-        {
-            double part[MAXC];
-#pragma unroll
-            for (int q = 0; q < MAXC; ++q) {
-                part[q] = 0.0;
-                float* slot = sm_boxes + (size_t)(g * MAXC + q) * SLOT;
-                const float* Pb = slot;
-                float* Apb = slot + kBZ;   // the p_{k-1} box is dead now: A p goes to its centre
-                const float* axb = slot + 2 * kBZ;
-                const float* ayb = axb + kBX;
-                const float* azb = ayb + kBY;
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const Cell cl = tile_cell(my[q], n, lt, m);
-                    if (!have[q] || !cl.ok) continue;
-                    const int bi = m, bj = lt >> 5, bk = lt & 31;
-                    const int o = (bi + 1) * 400 + (bj + 1) * 40 + (bk + 4);
-                    const float pc = Pb[o];
-                    float ap;
-                    if (HEAT) {
-                        // heat.py:94-105 with heat.py:55-91 neighbour_terms (use_fixed = 0): identity rows on fixed
-                        // cells, fixed neighbours enter as kappa_f x_c
-                        const unsigned char* flb = reinterpret_cast<const unsigned char*>(azb + kBW);
-                        const int of = (bi + 1) * 640 + (bj + 1) * 64 + (bk + 16);
-                        if (flb[of] & 1) {
-                            ap = pc;
-                        } else {
-                            float acc = 0.0f;
-                            float kf;
-                            if (cl.i > 0) {
-                                kf = axb[bi * 256 + bj * 32 + bk];
-                                acc = __fadd_rn(acc, (flb[of - 640] & 1) ? __fmul_rn(kf, pc) : __fmul_rn(kf, __fsub_rn(pc, Pb[o - 400])));
-                            }
-                            if (cl.i < n - 1) {
-                                kf = axb[(bi + 1) * 256 + bj * 32 + bk];
-                                acc = __fadd_rn(acc, (flb[of + 640] & 1) ? __fmul_rn(kf, pc) : __fmul_rn(kf, __fsub_rn(pc, Pb[o + 400])));
-                            }
-                            if (cl.j > 0) {
-                                kf = ayb[bi * 288 + bj * 32 + bk];
-                                acc = __fadd_rn(acc, (flb[of - 64] & 1) ? __fmul_rn(kf, pc) : __fmul_rn(kf, __fsub_rn(pc, Pb[o - 40])));
-                            }
-                            if (cl.j < n - 1) {
-                                kf = ayb[bi * 288 + (bj + 1) * 32 + bk];
-                                acc = __fadd_rn(acc, (flb[of + 64] & 1) ? __fmul_rn(kf, pc) : __fmul_rn(kf, __fsub_rn(pc, Pb[o + 40])));
-                            }
-                            if (cl.k > 0) {
-                                kf = azb[bi * 288 + bj * 36 + bk];
-                                acc = __fadd_rn(acc, (flb[of - 1] & 1) ? __fmul_rn(kf, pc) : __fmul_rn(kf, __fsub_rn(pc, Pb[o - 1])));
-                            }
-                            if (cl.k < n - 1) {
-                                kf = azb[bi * 288 + bj * 36 + bk + 1];
-                                acc = __fadd_rn(acc, (flb[of + 1] & 1) ? __fmul_rn(kf, pc) : __fmul_rn(kf, __fsub_rn(pc, Pb[o + 1])));
-                            }
-                            ap = __fadd_rn(pc, __fmul_rn(c_dt, acc));
-                        }
-                    } else {
-                        float acc = 0.0f;
-                        if (cl.i > 0) acc = __fadd_rn(acc, __fmul_rn(axb[bi * 256 + bj * 32 + bk], __fsub_rn(pc, Pb[o - 400])));
-                        if (cl.i < n - 1)
-                            acc = __fadd_rn(acc, __fmul_rn(axb[(bi + 1) * 256 + bj * 32 + bk], __fsub_rn(pc, Pb[o + 400])));
-                        if (cl.j > 0) acc = __fadd_rn(acc, __fmul_rn(ayb[bi * 288 + bj * 32 + bk], __fsub_rn(pc, Pb[o - 40])));
-                        if (cl.j < n - 1)
-                            acc = __fadd_rn(acc, __fmul_rn(ayb[bi * 288 + (bj + 1) * 32 + bk], __fsub_rn(pc, Pb[o + 40])));
-                        if (cl.k > 0) acc = __fadd_rn(acc, __fmul_rn(azb[bi * 288 + bj * 36 + bk], __fsub_rn(pc, Pb[o - 1])));
-                        if (cl.k < n - 1)
-                            acc = __fadd_rn(acc, __fmul_rn(azb[bi * 288 + bj * 36 + bk + 1], __fsub_rn(pc, Pb[o + 1])));
-                        ap = div_rn(acc, hhd);
-                    }
-                    Apb[o] = ap;
-                    pnew[cl.t] = pc;
-                    part[q] += (double)pc * (double)ap;
-                }
-            }
-            group_sum<MAXC>(part, red);
-#pragma unroll
-            for (int q = 0; q < MAXC; ++q) {
-                const int c = c0 + g + groups * q;
-                if (lt == 0 && have[q]) bufA[c] = part[q];
-            }
-        }
-        if (!grid_barrier(bar, epoch, ws.err, gridDim.x)) goto finish;
-        {
-            double tot[1];
-            const int comp[1] = {0};
-            scene_sums<1>(bufA, cb, ce, comp, tot, red, ws.tiles);
-            if (threadIdx.x == 0) {
-                Ls.pAp = tot[0];
-                Ls.alpha = __double2float_rn(Ls.rz / tot[0]);
-            }
-            __syncthreads();
-        }
-        // phase B: x += alpha p, r -= alpha Ap, z = D r; publish z; r.r and r.z
-        {
-            const float alpha = Ls.alpha;
-            double part[2 * MAXC];
-#pragma unroll
-            for (int q = 0; q < MAXC; ++q) {
-                part[2 * q] = part[2 * q + 1] = 0.0;
-                const float* slot = sm_boxes + (size_t)(g * MAXC + q) * SLOT;
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const int s = q * 4 + m;
-                    const Cell cl = tile_cell(my[q], n, lt, m);
-                    if (!have[q] || !cl.ok) continue;
-                    const int o = (m + 1) * 400 + ((lt >> 5) + 1) * 40 + ((lt & 31) + 4);
-                    x[s] = __fadd_rn(x[s], __fmul_rn(alpha, slot[o]));
-                    r[s] = __fsub_rn(r[s], __fmul_rn(alpha, slot[kBZ + o]));
-                    const float z = __fmul_rn(D[s], r[s]);
-                    zg[cl.t] = z;
-                    part[2 * q] += (double)r[s] * (double)r[s];
-                    part[2 * q + 1] += (double)r[s] * (double)z;
-                }
-            }
-            group_sum<2 * MAXC>(part, red);
-#pragma unroll
-            for (int q = 0; q < MAXC; ++q) {
-                const int c = c0 + g + groups * q;
-                if (lt == 0 && have[q]) {
-                    bufB[1 * ws.tiles + c] = part[2 * q];
-                    bufB[2 * ws.tiles + c] = part[2 * q + 1];
-                }
-            }
-        }
-        if (!grid_barrier(bar, epoch, ws.err, gridDim.x)) goto finish;
-        issue_boxes(kit + 1);
-        requested = true;
-        {
-            double tot[2];
-            const int comp[2] = {1, 2};
-            scene_sums<2>(bufB, cb, ce, comp, tot, red, ws.tiles);
-            if (threadIdx.x == 0) update_scalars(Ls, HEAT, tot[0], tot[1], kit);
-            __syncthreads();
-        }
-    }
-    if (requested) {
-        // the solve ended: the boxes requested for an iteration that does not run are waited for (no copy in flight)
-        bool ok = true;
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q)
-            if (have[q]) ok = mbar_wait(&mbar[g * MAXC + q], phase_bit) && ok;
-        if (!ok) atomicExch(ws.err, 1);
-        phase_bit ^= 1u;
-        requested = false;
-    }
-    // -------------------------------------------------- write x back, then (pressure) project the faces
-#pragma unroll
-    for (int q = 0; q < MAXC; ++q) {
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const Cell cl = tile_cell(my[q], n, lt, m);
-            if (have[q] && cl.ok) xg[cl.t] = x[q * 4 + m];
-        }
-    }
-    if (!HEAT) {
-        if (!grid_barrier(bar, epoch, ws.err, gridDim.x)) goto finish;
-        const float dtr = (float)(dt_d / S.rho);
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) {
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const Cell cl = tile_cell(my[q], n, lt, m);
-                if (have[q] && cl.ok)
-                    project_cell(S, S.u[par ^ 1], S.v[par ^ 1], S.w[par ^ 1], S.p, x[q * 4 + m], dtr, h, cl);
-            }
-        }
-    }
-finish:
-    if (*(volatile int*)ws.err) {
-        // leave no copy in flight: a timed-out wait is retried (bounded) before the block exits
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q)
-            if (have[q]) mbar_wait(&mbar[g * MAXC + q], phase_bit ^ 1u);
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) write_stats(S, Ls, HEAT, *(volatile int*)ws.err != 0, par);
-}
-
 // ===================================================== resident pressure CG, one reduction point per iteration
 // Jacobi-PCG of the pressure system of one scene (n % 4 == 0) with ONE grid barrier per iteration instead of two.  The
 // vectors follow the classic recurrences (A p formed from p every iteration, r -= alpha A p, p = z + beta p with
@@ -2232,35 +1476,10 @@ const void* pcg_kernel(bool heat, bool tma) {
 
 size_t pcg_stream_smem(bool tma) { return tma ? 2 * (size_t)kSlotFloats * sizeof(float) + 128 : 0; }
 
-const void* pcg_resident_kernel(bool heat, int maxc, bool tma) {
-    if (heat && tma) {
-        if (maxc == 1) return (const void*)k_pcg_tma<true, 1>;
-        if (maxc == 2) return (const void*)k_pcg_tma<true, 2>;
-        return (const void*)k_pcg_tma<true, 3>;
-    }
-    if (heat) {
-        if (maxc == 1) return (const void*)k_pcg_res<true, 1, false>;
-        if (maxc == 2) return (const void*)k_pcg_res<true, 2, false>;
-        return (const void*)k_pcg_res<true, 3, false>;
-    }
-    if (tma) {
-        if (maxc == 1) return (const void*)k_pcg_tma<false, 1>;
-        if (maxc == 2) return (const void*)k_pcg_tma<false, 2>;
-        return (const void*)k_pcg_tma<false, 3>;
-    }
-    if (maxc == 1) return (const void*)k_pcg_res<false, 1, false>;
-    if (maxc == 2) return (const void*)k_pcg_res<false, 2, false>;
-    return (const void*)k_pcg_res<false, 3, false>;
-}
-
 int set_wait_limit(unsigned long long limit_ns, int absent_block) {
     if (cudaMemcpyToSymbol(c_wait_limit_ns, &limit_ns, sizeof limit_ns) != cudaSuccess) return HF_ERR_CUDA;
     if (cudaMemcpyToSymbol(c_absent_block, &absent_block, sizeof absent_block) != cudaSuccess) return HF_ERR_CUDA;
     return brick_set_wait_limit(limit_ns, absent_block);
-}
-
-size_t pcg_resident_smem(int groups, int maxc, bool tma, bool heat) {
-    return tma ? (size_t)groups * maxc * (heat ? kHeatSlotFloats : kSlotFloats) * sizeof(float) + 128 : 0;
 }
 
 }  // namespace hf

@@ -42,7 +42,8 @@ __device__ __forceinline__ Cell tile_cell(const TileItem& ti, int n, int lt, int
 constexpr int kUnits = 148;
 
 __host__ __device__ inline int unit_count(int tiles) { return tiles < kUnits ? tiles : kUnits; }
-__host__ __device__ inline int unit_first(int tiles, int units, int u) { return (int)((long long)tiles * u / units); }
+// (32-bit arithmetic: units are formed of at most kUnits * kBrickWideTiles tiles)
+__host__ __device__ inline int unit_first(int tiles, int units, int u) { return tiles * u / units; }
 
 // Per-block copy of a scene's CG scalars; every block derives them from the same partial sums, so all copies agree.
 struct LocalScene {

@@ -53,7 +53,7 @@ struct BrickLaunch {
 };
 // the kernel for such blocks and its threads: (const hf_scene*, const TileItem*, double dt, Workspace, BrickLaunch), dynamic
 // shared memory brick_smem(...)
-const void* brick_kernel(const BrickLaunch& bl, int* threads);
+const void* brick_kernel(const BrickLaunch& bl, bool heat, int* threads);
 size_t brick_smem(const BrickLaunch& bl);
 int brick_box_bytes();
 int brick_set_wait_limit(unsigned long long limit_ns, int absent_block);
@@ -63,9 +63,7 @@ size_t streaming_workspace_bytes(int num_scenes, int num_chunks, int num_tiles);
 // TMA descriptors of the tiled pressure stencil (resident CG): z, both search-direction buffers, alpha_f x (the u
 // lattice), and the cell-layout copies of alpha_f y and z.
 struct TileMaps {
-    CUtensorMap z, p0, p1, ax, ayc, azc;      // pressure (and the z / p boxes of the heat system)
-    CUtensorMap hkx, hky, hkzc, flags;        // heat: face diffusivities and the cell flags (bytes)
-    CUtensorMap t0, t1;                       // heat: both temperature buffers (x0 is the one the parity selects)
+    CUtensorMap z, p0, p1, ax, ayc, azc;
 };
 
 __global__ void k_scatter(const hf_scene* __restrict__ scenes, int s);
@@ -98,11 +96,6 @@ __global__ void k_heat_matvec_plain(int n, float h, float dt, float alpha, float
 const void* pcg_kernel(bool heat, bool tma);
 // dynamic shared memory of the streaming kernel (tma: one stencil slot per block, staged with TMA)
 size_t pcg_stream_smem(bool tma);
-// register-resident single-scene variant (MAXC tiles per 256-thread group: 1, 2 or 3; blockDim = 256 x groups);
-// arguments: (const hf_scene*, const TileItem*, int tile_lo, int tile_hi, double dt, Workspace, TileMaps) -- the
-// scene's tiles; the TileMaps is used when tma; dynamic shared memory pcg_resident_smem(...)
-const void* pcg_resident_kernel(bool heat, int maxc, bool tma);
-size_t pcg_resident_smem(int groups, int maxc, bool tma, bool heat);
 // single-reduction register-resident pressure solve of one scene with n % 4 == 0 (one grid barrier per CG iteration;
 // uses hdiag as scratch), the same arguments and thread layout as the TMA resident variant; dynamic shared memory
 // pcg_one_smem(groups, maxc)
