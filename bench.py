@@ -75,8 +75,8 @@ def parse():
     ap.add_argument("--persistent-blocks", type=int, default=0, help="plain: grid of the streaming CG kernel")
     ap.add_argument("--no-tma", action="store_true", help="plain: resident pressure CG without the TMA-staged stencil")
     ap.add_argument("--cg", default="single-reduction", choices=["classic", "single-reduction"],
-                    help="plain: pressure solve by the classic Jacobi-PCG or its single-reduction form (one grid "
-                         "barrier per iteration)")
+                    help="plain: the pressure solve that HeatflowMPM is asked for (both are served by the on-chip classic "
+                         "Jacobi-PCG)")
     ap.add_argument("--scenes", type=int, default=64, help="batched: scenes in the ensemble")
     ap.add_argument("--graph-steps", type=int, default=10, help="batched: substeps per captured CUDA graph")
     ap.add_argument("--edges", default="32,48,64,96,128", help="batched: grid edges the ensemble draws from")
@@ -496,16 +496,13 @@ def bench_plain(args, dev, rank, world, local):
     peaks = load_peaks()
     cg_bytes = pressure_bytes_per_launch(N, p_iters / steps)
     traffic = None
-    single = args.cg == "single-reduction"
     try:
-        prof = json.load(open(os.path.join(ROOT, "profiles", "pressure_cg_one_96.json" if single else "pressure_cg_96.json")))
+        prof = json.load(open(os.path.join(ROOT, "profiles", "pressure_cg_chip_96.json")))
         traffic = prof["dram_bytes_per_iteration"] * (p_iters / steps) + prof.get("dram_bytes_fixed", 0.0)
     except (OSError, ValueError, KeyError):
         pass
-    kernel = ("k_pcg_one<3> (single-reduction pressure Jacobi-PCG + projection: one grid barrier per iteration, one "
-              "persistent cooperative launch, TMA-staged register-resident stencil)" if single else
-              "k_pcg_tma<2> (pressure Jacobi-PCG + projection, one persistent cooperative launch, TMA-staged "
-              "register-resident stencil)")
+    kernel = ("k_brick<3, 2, false> (pressure Jacobi-PCG + projection, one persistent cooperative launch, CG state in registers "
+              "and shared memory, tagged exchanges)")
     roof = roofline(cg_bytes / (cg_ms / steps / 1000.0) / 1e9, peaks, traffic=traffic, kernel=kernel,
                     bytes_per_launch=cg_bytes, ms_per_launch=cg_ms / steps, mean_pressure_iters=p_iters / steps)
     sb = substep_bytes(N, h_iters / steps, p_iters / steps, True)
@@ -689,7 +686,7 @@ def bench_batched(args, dev, rank, world, local, steps, warmup, cpu_sample=True)
                    for s, a, b in zip(mine, sa, sbk))
     peaks = load_peaks()
     roof = roofline(cg_bytes / (cg_ms / 1000.0) / 1e9, peaks, traffic=None,
-                    kernel="k_pcg<false, true> (streaming persistent pressure Jacobi-PCG + projection over the scene table, TMA-staged double-buffered tile boxes)",
+                    kernel="k_brick<3, 5, false> (pressure Jacobi-PCG + projection, one team of blocks per scene, CG state on the chip)",
                     bytes_per_launch=cg_bytes, ms_per_launch=cg_ms, measured_on="rank 0 stage breakdown, 10 substeps")
     sub_gbs = sb / (el_ms / steps / 1000.0) / 1e9
     # ---- end to end through the public API: AirBatch.substep per substep, every scene's status block read back

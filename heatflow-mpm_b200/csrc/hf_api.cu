@@ -39,13 +39,8 @@ struct DeviceInfo {
     int occ_heat = 0, occ_pressure = 0, occ_pressure_tma = 0;
     size_t smem_optin = 0;
     bool ready = false;
-    // occupancy of the single-reduction pressure variant [tiles per group][groups] (-1: not queried yet; the query also
-    // raises the kernel's dynamic shared-memory limit)
-    int pipe_occ[4][5];
     bool brick_ready[3][hf::kBrickWideTiles + 1];  // the on-chip pressure solve's kernels whose shared-memory limit is raised
 };
-
-constexpr int kResGroupsMax[4] = {0, 4, 3, 2};   // 256-thread groups per block of the single-reduction variant, by MAXC
 
 std::mutex g_mu;
 DeviceInfo g_dev[64];
@@ -81,7 +76,6 @@ int device_info(DeviceInfo** out) {
         HF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "cudaDeviceGetAttribute");
         d.smem_optin = (size_t)optin;
         if (!d.coop) return fail(HF_ERR_DEVICE, "device does not support cooperative launches");
-        std::memset(d.pipe_occ, 0xff, sizeof d.pipe_occ);
         std::memset(d.brick_ready, 0, sizeof d.brick_ready);
         d.ready = true;
     }
@@ -110,10 +104,10 @@ Layout layout(int S, int C, int T) {
     o = align_up(o + sizeof(int) * (size_t)(S + 1), 256);
     L.maps = o;                      // kMapsPerScene TMA descriptors per scene (128 bytes each)
     o = align_up(o + sizeof(CUtensorMap) * hf::kMapsPerScene * (size_t)S, 256);
-    L.partA = o;                     // 5 doubles per tile, component-major (3 components used by the classic variants)
-    o = align_up(o + sizeof(double) * 5 * (size_t)T, 256);
+    L.partA = o;                     // 3 doubles per tile, component-major
+    o = align_up(o + sizeof(double) * 3 * (size_t)T, 256);
     L.partB = o;
-    o = align_up(o + sizeof(double) * 5 * (size_t)T, 256);
+    o = align_up(o + sizeof(double) * 3 * (size_t)T, 256);
     L.mean_part = o;
     o = align_up(o + sizeof(double) * (size_t)C, 256);
     L.streaming = o;
@@ -177,10 +171,8 @@ int encode_map(CUtensorMap* m, const float* base, int nk, int nj, int ni, int bk
     return HF_OK;
 }
 
-// The six TMA descriptors of a scene's tiled pressure stencil (order of hf::TileMaps): z and both search-direction
-// buffers with a one-cell halo, alpha_f x on its face lattice, alpha_f y and z in cell layout.
-static_assert(sizeof(hf::TileMaps) == 6 * sizeof(CUtensorMap), "TileMaps is six consecutive descriptors");
-
+// The six TMA descriptors of a scene's tiled pressure stencil: z and both search-direction buffers with a one-cell halo,
+// alpha_f x on its face lattice, alpha_f y and z in cell layout.
 int encode_scene_maps(const hf_scene& sc, CUtensorMap* m) {
     const int n = sc.n;
     int rc;
@@ -332,56 +324,6 @@ int launch_brick(const hf_plan* p, DeviceInfo* d, bool heat, double dt, void* st
     return HF_OK;
 }
 
-// The single-reduction pressure solve of a plan with one active scene (n % 4 == 0) whose tiles fit one block per SM.
-// Returns HF_OK after launching, or -1 when it does not apply (the caller falls back to the classic solves).
-int launch_one(const hf_plan* p, DeviceInfo* d, double dt, int s, void* stream) {
-    hf::Workspace ws = workspace(p);
-    const hf_scene* scenes = static_cast<const hf_scene*>(p->scenes_dev);
-    const hf::TileItem* tiles = static_cast<const hf::TileItem*>(p->tiles_dev);
-    const hf_scene& sc = p->scenes_host[s];
-    int t_lo = 0, t_hi = p->num_tiles, rc;
-    const int nt = t_hi - t_lo;
-    const int G = nt < d->sms ? nt : d->sms;
-    const int tpb = (nt + G - 1) / G;
-    // its stencil boxes are staged by TMA (16-byte float rows) and its scratch vectors must exist
-    if ((p->options & HF_PLAN_NO_TMA) || sc.n % 4 != 0 || !sc.cg_r || !sc.cg_z || !sc.cg_Ap || !sc.hdiag || !sc.pdiag ||
-        !sc.cg_p[0] || !sc.cg_p[1])
-        return -1;
-    const int want = (int)((p->options >> HF_PLAN_RES_TILES_SHIFT) & 3u);   // 0: the first that fits
-    // tiles per group: three first (two 256-thread groups of 128 registers per thread: the per-thread state does not fit
-    // the 80 registers of a 768-thread block), unless the block has few
-    const bool three_first = !want && tpb > 4;
-    for (int mi = 0; mi < 3; ++mi) {
-        const int m = want ? want + mi : (three_first ? 3 - mi : 1 + mi);
-        if (m > 3) break;
-        const int groups = (tpb + m - 1) / m;
-        if (groups > kResGroupsMax[m]) continue;
-        // one set of partials per 256-thread group into buffers sized by tiles
-        if (G * groups > nt) continue;
-        const void* fn = hf::pcg_one_kernel(m);
-        const size_t smem = hf::pcg_one_smem(groups, m);
-        if (smem > d->smem_optin) continue;
-        int& occ = d->pipe_occ[m][groups];
-        if (occ < 0) {
-            if (smem > 48 * 1024)
-                HF_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attribute");
-            int o = 0;
-            HF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, 256 * groups, smem), "occupancy (single-reduction)");
-            occ = o;
-        }
-        if (occ < 1) continue;
-        hf::TileMaps maps;
-        std::memset(&maps, 0, sizeof maps);
-        if ((rc = encode_scene_maps(sc, &maps.z))) return rc;
-        HF_CUDA(cudaMemsetAsync(ws.bar, 0, kHeadBytes, S(stream)), "cudaMemsetAsync(barrier)");
-        void* args[] = {(void*)&scenes, (void*)&tiles, (void*)&t_lo, (void*)&t_hi, (void*)&dt, (void*)&ws, (void*)&maps};
-        HF_CUDA(cudaLaunchCooperativeKernel(fn, dim3(G), dim3(256 * groups), args, smem, S(stream)),
-                "cooperative launch (single-reduction CG)");
-        return HF_OK;
-    }
-    return -1;
-}
-
 // Both CG solves of a plan.  The on-chip solve where every active scene fits it.  Otherwise one launch of the
 // streaming kernel: the active scenes are cut, in table order, into groups of at most kGroupScenes scenes and
 // group_cells cells (default kGroupCells: a group's CG vectors stay in L2), solved by the lanes of the grid.
@@ -390,22 +332,17 @@ int launch_pcg(const hf_plan* p, bool heat, double dt, void* stream) {
     int rc = device_info(&d);
     if (rc) return rc;
     if (p->num_tiles == 0) return HF_OK;
-    int nactive = 0, last = -1, total = 0;
+    int nactive = 0, total = 0;
     bool correction = false;   // the outer defect correction runs in the streaming kernel only
     for (int s = 0; s < p->num_scenes; ++s)
         if (p->scenes_host[s].flags & HF_FLAG_ACTIVE) {
             ++nactive;
-            last = s;
             total += tiles_of(p->scenes_host[s].n);
             correction = correction || (p->scenes_host[s].flags & HF_FLAG_DEFECT_CORRECTION);
         }
     if (total != p->num_tiles) return fail(HF_ERR_ARG, "plan changed since hf_plan_upload");
     if (nactive > 0 && !correction && !(p->options & HF_PLAN_STREAMING_CG) &&
         !(heat && nactive == 1 && (p->options & HF_PLAN_STREAMING_HEAT))) {
-        if (!heat && nactive == 1 && (p->options & HF_PLAN_SINGLE_REDUCTION_CG)) {
-            rc = launch_one(p, d, dt, last, stream);
-            if (rc != -1) return rc;
-        }
         rc = launch_brick(p, d, heat, dt, stream);
         if (rc != -1) return rc;
     }

@@ -19,20 +19,18 @@
 // Two grid barriers per iteration: the search direction p_k = z + beta p_{k-1} is not a separate phase -- every block
 // recomputes it at the stencil points it reads from z and the previous p (double-buffered), so it costs no barrier.
 //
-// Variants (the on-chip solves of hf_brick.cu take the plans whose scenes fit there; these take the rest):
-//   k_pcg       streaming: vectors in global memory, any number of scenes.  The scenes come
-//               in L2-sized groups solved by the lanes of the grid; for the pressure system with every scene at
-//               n % 4 == 0 each tile's stencil boxes and CG vectors are staged by TMA from per-scene descriptors,
-//               double-buffered per block.  Optional outer defect correction (fp64 true residual, restart).
-//   k_pcg_one   pressure solve of one scene with n % 4 == 0 with one grid barrier per iteration (see there).
+// k_pcg streams: the vectors stay in global memory, for any number of scenes of any size (the on-chip solves of hf_brick.cu
+// take the plans whose scenes fit there).  The scenes come in L2-sized groups solved by the lanes of the grid; for the
+// pressure system with every scene at n % 4 == 0 each tile's stencil boxes and CG vectors are staged by TMA from
+// per-scene descriptors, double-buffered per block.  Optional outer defect correction (fp64 true residual, restart).
 #include <cuda.h>
 
 #include "hf_cg.cuh"
 
 namespace hf {
 
-// Components one group_sum / scene_sums call reduces at most: 3 inner products per tile x 3 tiles of a 256-thread
-// group (the resident variants' set-up).  Every CG kernel's `red` holds kRedComps x 32 doubles (one per warp).
+// k_pcg's `red` holds kRedComps x 32 doubles: up to 9 components of one sum, or the 8 warps' sums of the group_sums of 36
+// scenes and one component.
 constexpr int kRedComps = 9;
 constexpr int kMaxCorrections = 2;   // restarts of one solve by the outer defect correction
 
@@ -202,120 +200,6 @@ __device__ __forceinline__ void group_sum(double (&v)[K], double* red) {
     }
 }
 
-// group_sum in two steps, so that a thread holds the partials of one tile at a time: stash_warp reduces K values over the
-// warp (the same butterfly) and lane 0 parks them in red[(c0 + c) * 32 + warp]; after every tile's stash,
-// publish_group (thread lt == 0 of each 256-thread group) adds the group's 8 warps in order -- group_sum's tree, the
-// same bits -- and writes the tile partials to buf[c * tiles + tile] (3 components, component-major).  red must not be read by
-// another phase in between (the caller's barriers see to that).
-template <int K>
-__device__ __forceinline__ void stash_warp(double (&v)[K], double* red, int c0) {
-#pragma unroll
-    for (int c = 0; c < K; ++c) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int c = 0; c < K; ++c) red[(c0 + c) * 32 + (threadIdx.x >> 5)] = v[c];
-    }
-}
-
-template <int MAXC>
-__device__ __forceinline__ void publish_group(const double* red, double* __restrict__ buf, int first_tile, int groups,
-                                              int c_end, int tiles) {
-    __syncthreads();
-    if ((threadIdx.x & 255) == 0) {
-        const int g0 = (threadIdx.x >> 5);   // first warp of this group
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) {
-            const int c = first_tile + groups * q;
-            if (c >= c_end) continue;
-#pragma unroll
-            for (int comp = 0; comp < 3; ++comp) {
-                double s = 0.0;
-#pragma unroll
-                for (int w = 0; w < 8; ++w) s += red[(3 * q + comp) * 32 + g0 + w];
-                buf[comp * tiles + c] = s;
-            }
-        }
-    }
-}
-
-// One partial per 256-thread group (the single-reduction CG's five components), stored component-major so that a
-// warp's loads of one component are contiguous: after stash_warp<K>(v, red, 0) in every warp, thread lt == 0 of each
-// group adds its 8 warps in order and writes buf[comp * units + unit].
-template <int K>
-__device__ __forceinline__ void publish_unit(const double* red, double* __restrict__ buf, int unit, int units) {
-    __syncthreads();
-    if ((threadIdx.x & 255) == 0) {
-        const int g0 = (threadIdx.x >> 5);
-#pragma unroll
-        for (int comp = 0; comp < K; ++comp) {
-            double s = 0.0;
-#pragma unroll
-            for (int w = 0; w < 8; ++w) s += red[comp * 32 + g0 + w];
-            buf[comp * units + unit] = s;
-        }
-    }
-}
-
-// The K sums of the groups' component-major partials (publish_unit), in every thread of the block.  The tree is
-// scene_sums_3g's: the G groups of 256 threads take components q, q + G, ...; thread lt adds units lt, lt + 256, ...
-// in order (absent ones as +0.0), then the warp butterfly and the 8 warps in order.  unit_loads issues the loads of
-// the thread's first U units (so that the caller can put them ahead of other memory traffic); unit_sums adds them,
-// then any further units, and reduces.
-template <int K, int G, int U>
-__device__ __forceinline__ void unit_loads(const double* __restrict__ buf, int units, double (&v)[K][U]) {
-    constexpr int KPT = (K + G - 1) / G;
-    const int q = threadIdx.x >> 8, lt = threadIdx.x & 255;
-#pragma unroll
-    for (int j = 0; j < KPT; ++j)
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            v[j][u] = q < G && q + G * j < K && lt + u * kThreads < units ? buf[(q + G * j) * units + lt + u * kThreads] : 0.0;
-}
-
-template <int K, int G, int U>
-__device__ __forceinline__ void unit_sums(const double* __restrict__ buf, int units, const double (&v)[K][U],
-                                          double (&tot)[K], double* red) {
-    constexpr int KPT = (K + G - 1) / G;
-    const int q = threadIdx.x >> 8, lt = threadIdx.x & 255;
-    double acc[KPT];
-#pragma unroll
-    for (int j = 0; j < KPT; ++j) {
-        acc[j] = 0.0;
-#pragma unroll
-        for (int u = 0; u < U; ++u) acc[j] += v[j][u];
-    }
-    if (q < G) {
-        for (int c = lt + U * kThreads; c < units; c += kThreads) {
-#pragma unroll
-            for (int j = 0; j < KPT; ++j)
-                if (q + G * j < K) acc[j] += buf[(q + G * j) * units + c];
-        }
-#pragma unroll
-        for (int j = 0; j < KPT; ++j) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
-        }
-    }
-    const int lane = threadIdx.x & 31, wq = lt >> 5;
-    __syncthreads();
-    if (q < G && lane == 0) {
-#pragma unroll
-        for (int j = 0; j < KPT; ++j)
-            if (q + G * j < K) red[(q + G * j) * 32 + wq] = acc[j];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int c = 0; c < K; ++c) {
-        double s = 0.0;
-#pragma unroll
-        for (int w = 0; w < kThreads / 32; ++w) s += red[c * 32 + w];
-        tot[c] = s;
-    }
-}
-
 // Search direction at cell t for iteration k: p_k = z + beta p_{k-1} (warp's _cg_kernel_2), or z at k = 1.
 struct Dir {
     const float* z;
@@ -325,11 +209,6 @@ struct Dir {
     __device__ __forceinline__ float operator()(int t) const {
         return first ? z[t] : __fadd_rn(z[t], __fmul_rn(beta, pold[t]));
     }
-};
-
-struct Vec {
-    const float* a;
-    __device__ __forceinline__ float operator()(int t) const { return a[t]; }
 };
 
 // grid.py:94-115 k_laplacian accumulation, the sum over the six faces of alpha_f (x_c - x_nb) with domain faces skipped,
@@ -1051,424 +930,6 @@ __global__ void __launch_bounds__(kThreads) k_pcg(const hf_scene* __restrict__ s
                 if (scenes[s].flags & HF_FLAG_ACTIVE) scenes[s].state->status |= HF_SCENE_BARRIER_TIMEOUT;
     }
 }
-
-// ===================================================== resident pressure CG, one reduction point per iteration
-// Jacobi-PCG of the pressure system of one scene (n % 4 == 0) with ONE grid barrier per iteration instead of two.  The
-// vectors follow the classic recurrences (A p formed from p every iteration, r -= alpha A p, p = z + beta p with
-// z ~ D r); only beta is obtained differently.  In iteration k every block forms, next to p_k . A p_k, the direct
-// r_k . r_k and r_k . z_k of its cells and the two terms A p_k . z_k and A p_k . D A p_k, so that one scene sum gives
-//     alpha_k = rz_k / pAp_k,   rz_{k+1} = rz_k - 2 alpha_k (A p_k . z_k) + alpha_k^2 (A p_k . D A p_k),
-//     beta_{k+1} = rz_{k+1} / rz_k
-// (the expansion of (r_k - alpha A p_k) . D (r_k - alpha A p_k) used by D'Azevedo, Eijkhout & Romine, "Conjugate
-// gradient algorithms with reduced synchronization overhead on distributed memory multiprocessors", 1993).  rz_k is
-// the direct sum of every iteration, so the expansion never accumulates; it differs from the direct rz_{k+1} only by
-// the binary32 rounding of r_{k+1} (~1e-7 relative), so beta moves by that much and the solve converges like the
-// classic one (the same iteration counts and x within ~1e-8 relative on the benchmark scene's systems; at tolerance
-// 1e-6 too).  The convergence test is the classic one on the direct r_k . r_k, taken at the barrier after r_k was
-// formed: a solve stops with the same x and reports the same iteration count.
-//
-// Partials: a thread adds the five products of its cells in cell order, the warp butterfly and the group's 8 warps in
-// order give one set per 256-thread group, and every block sums the groups' sets in group order (the set-up's three
-// sums stay per tile).  The tree is fixed for a given grid, so a solve is deterministic; unlike the classic variants'
-// per-tile tree it depends on the launch shape (this kernel only runs single-scene plans).
-//
-// Halo: iteration k + 1 needs p_{k+1} = z_{k+1} + beta p_k at the tile's face neighbours, which belong to other
-// blocks.  Every block publishes, for the cells on its tiles' faces, z_k' = D r_k and q_k = D A p_k (double-buffered:
-// z' in cg_r / cg_z, q in cg_Ap / hdiag -- the heat diagonal is dead while the pressure system is solved).  Right
-// after the barrier a block requests the z', q values of its tiles' 832 face-neighbour points (cp.async), in flight
-// while it sums the partials; then every p_{k+1} in its boxes, own cells and neighbours alike, is formed by the same
-// operations from the same values, z = z' - alpha q, p = z + beta p, so all blocks agree bit for bit and no block
-// needs another's p: the p boxes (one-cell halo) are loaded once, from the published p0 (TMA), and advanced in place.
-// State: r, A p and D of a thread's cells in registers; x, the p box, the face-fraction boxes (TMA, once) and the
-// halo staging in shared memory.
-constexpr int kOneFaces = kBZ;                            // slot offset of the face-fraction boxes
-constexpr int kOneCells = kBZ + kBX + kBY + kBW;          // slot offset of x (1024 floats)
-constexpr int kOneHalo = kOneCells + 1024;                // slot offset of the halo staging: z' and q of 832 points
-constexpr int kOneHaloPts = 832;
-constexpr int kOneSlotFloats = kOneHalo + 2 * kOneHaloPts;   // 8672 floats = 34,688 bytes (a multiple of 128)
-constexpr int kOneComps = 5;                              // partials per group: pAp, rr, rz, Ap.z, Ap.D.Ap
-static_assert(kOneSlotFloats % 32 == 0, "slots stay 128-byte aligned");
-
-// grid.py:94-115 k_laplacian of one tile cell from a staged box (centre offset o) and the tile's face boxes
-__device__ __forceinline__ float lap_box(const float* __restrict__ B, const float* __restrict__ axb,
-                                         const float* __restrict__ ayb, const float* __restrict__ azb, const Cell& cl,
-                                         int n, int bi, int bj, int bk, int o, const DivBy& hh) {
-    const float pc = B[o];
-    float acc = 0.0f;
-    if (cl.i > 0) acc = __fadd_rn(acc, __fmul_rn(axb[bi * 256 + bj * 32 + bk], __fsub_rn(pc, B[o - 400])));
-    if (cl.i < n - 1) acc = __fadd_rn(acc, __fmul_rn(axb[(bi + 1) * 256 + bj * 32 + bk], __fsub_rn(pc, B[o + 400])));
-    if (cl.j > 0) acc = __fadd_rn(acc, __fmul_rn(ayb[bi * 288 + bj * 32 + bk], __fsub_rn(pc, B[o - 40])));
-    if (cl.j < n - 1) acc = __fadd_rn(acc, __fmul_rn(ayb[bi * 288 + (bj + 1) * 32 + bk], __fsub_rn(pc, B[o + 40])));
-    if (cl.k > 0) acc = __fadd_rn(acc, __fmul_rn(azb[bi * 288 + bj * 36 + bk], __fsub_rn(pc, B[o - 1])));
-    if (cl.k < n - 1) acc = __fadd_rn(acc, __fmul_rn(azb[bi * 288 + bj * 36 + bk + 1], __fsub_rn(pc, B[o + 1])));
-    return div_rn(acc, hh);
-}
-
-// Face-neighbour point u (0..3) of thread lt around a 4 x 8 x 32 tile, as box offsets (bi, bj, bk in -1..4, -1..8,
-// -1..32): the two i faces (256 points each), the two j faces (128 each) and the two k faces (32 each) -- 832 points,
-// three or four per thread, consecutive threads on consecutive k; staging index u * 256 + lt.  False when the thread
-// has no point u.
-__device__ __forceinline__ bool halo_point(int lt, int u, int& bi, int& bj, int& bk) {
-    if (u == 0 || u == 1) {
-        bi = u == 0 ? -1 : 4;
-        bj = lt >> 5;
-        bk = lt & 31;
-        return true;
-    }
-    if (u == 2) {
-        bi = (lt & 127) >> 5;
-        bj = lt < 128 ? -1 : 8;
-        bk = lt & 31;
-        return true;
-    }
-    if (lt >= 64) return false;
-    bi = (lt & 31) >> 3;
-    bj = lt & 7;
-    bk = lt < 32 ? -1 : 32;
-    return true;
-}
-
-// global cell of face-neighbour point u of thread lt around tile ti, or -1 (no point, or outside the domain)
-__device__ __forceinline__ int halo_cell(const TileItem& ti, int n, int lt, int u) {
-    int bi = 0, bj = 0, bk = 0;
-    if (!halo_point(lt, u, bi, bj, bk)) return -1;
-    const int gi = ti.i0 + bi, gj = ti.j0 + bj, gk = ti.k0 + bk;
-    if (gi < 0 || gi >= n || gj < 0 || gj >= n || gk < 0 || gk >= n) return -1;
-    return (gi * n + gj) * n + gk;
-}
-
-__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-
-template <int MAXC>
-__global__ void __launch_bounds__(MAXC == 1 ? 1024 : (MAXC == 2 ? 768 : 512), 1)
-    k_pcg_one(const hf_scene* __restrict__ scenes, const TileItem* __restrict__ tiles, int tile_lo, int tile_hi,
-              double dt_d, Workspace ws, const __grid_constant__ TileMaps maps) {
-    constexpr int CPT = 4 * MAXC;
-    extern __shared__ __align__(128) float sm_raw[];
-    float* sm_slots = align128_shared(sm_raw);
-    __shared__ double red[kOneComps * 3 * 32];   // five partials per warp (the set-up: three of up to three tiles)
-    __shared__ unsigned hmask_s[1024];
-    __shared__ TileItem my_s[4 * 3];
-    __shared__ LocalScene Ls;
-    __shared__ __align__(8) unsigned long long mbar[4 * 3];
-    const int groups = blockDim.x >> 8, g = threadIdx.x >> 8, lt = threadIdx.x & 255;
-    const int c0 = tile_lo + (int)(((long long)(tile_hi - tile_lo) * blockIdx.x) / gridDim.x);
-    const int c1 = tile_lo + (int)(((long long)(tile_hi - tile_lo) * (blockIdx.x + 1)) / gridDim.x);
-    const int sidx = tiles[c0].scene;
-    const hf_scene& S = scenes[sidx];
-    const int n = S.n, N = n * n * n;
-    const int par = S.state->parity;
-    unsigned* bar = ws.bar + kMaxLanes;
-    unsigned epoch = 0;
-    const float h = (float)S.h, hh = __fmul_rn(h, h);
-    const DivBy hhd = div_by(hh);
-    double* const bufA = ws.partA;
-    double* const bufB = ws.partB;
-    const int cb = ws.tile_begin[sidx], ce = ws.tile_begin[sidx + 1];
-    // the iterations' partials: one per 256-thread group, unit = block x groups + group (the launch keeps the units
-    // within the tile count that the partial buffers are sized for)
-    const int units = (int)gridDim.x * groups, unit = (int)blockIdx.x * groups + g;
-    float* xg = S.p;
-    // the group's tiles (shared memory, like the halo mask below: registers held through the solve make the stencil
-    // phase spill)
-    TileItem* const my = my_s + g * MAXC;
-    bool have[MAXC];
-#pragma unroll
-    for (int q = 0; q < MAXC; ++q) have[q] = c0 + g + groups * q < c1;
-    if (lt < MAXC) {
-        const int c = c0 + g + groups * lt;
-        my[lt] = tiles[c < c1 ? c : c0];
-    }
-    auto slot_of = [&](int q) { return sm_slots + (size_t)(g * MAXC + q) * kOneSlotFloats; };
-    unsigned phase_bit = 0;
-    auto wait_boxes = [&]() {
-        bool ok = true;
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q)
-            if (have[q]) ok = mbar_wait(&mbar[g * MAXC + q], phase_bit) && ok;
-        if (!ok) atomicExch(ws.err, 1);
-        phase_bit ^= 1u;
-    };
-    if (lt == 0) {
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) mbar_init(&mbar[g * MAXC + q], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    // bit 4 q + u of hmask_s[thread]: the thread's face-neighbour point u of tile q exists and lies in the domain
-    {
-        unsigned hm = 0;
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q)
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (have[q] && halo_cell(my[q], n, lt, u) >= 0) hm |= 1u << (4 * q + u);
-        hmask_s[threadIdx.x] = hm;
-    }
-    float r[CPT], ap[CPT], dg[CPT];
-    int k = 0;
-    // ------------------------------------------------------------------------------------------ set-up
-    float mean = 0.0f;
-    {
-        double mm[1];
-        const int comp[1] = {0};
-        scene_sums<1>(ws.mean_part, ws.chunk_begin[sidx], ws.chunk_begin[sidx + 1], comp, mm, red, 0);
-        mean = __double2float_rn(mm[0] / ((double)n * n * n));
-    }
-    {
-        // r0 = b - A x0, p0 = z0 = D r0 (published for the halo of A p0); partials b.b, r.r, r.z
-        __syncthreads();   // red is free (the rhs mean above read it)
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) {
-            double part[3] = {0.0, 0.0, 0.0};
-            float* X = slot_of(q) + kOneCells;
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const int s = q * 4 + m, e = m * 256 + lt;
-                r[s] = ap[s] = dg[s] = 0.0f;
-                X[e] = 0.0f;
-                const Cell cl = tile_cell(my[q], n, lt, m);
-                if (!have[q] || !cl.ok) continue;
-                float b, d, rr;
-                setup_cell<false>(S, xg, mean, hh, 0.0f, cl, b, d, rr);
-                const float z = __fmul_rn(d, rr);
-                X[e] = xg[cl.t];
-                dg[s] = d;
-                r[s] = rr;
-                S.cg_p[0][cl.t] = z;
-                part[0] += (double)b * (double)b;
-                part[1] += (double)rr * (double)rr;
-                part[2] += (double)rr * (double)z;
-            }
-            stash_warp<3>(part, red, 3 * q);
-        }
-        publish_group<MAXC>(red, bufB, c0 + g, groups, c1, ws.tiles);
-    }
-    // the tiles' face fractions stay in shared memory for the whole solve
-    if (lt == 0) {
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) {
-            if (!have[q]) continue;
-            float* slot = slot_of(q);
-            unsigned long long* mb = &mbar[g * MAXC + q];
-            mbar_expect_tx(mb, (unsigned)((kBX + kBY + kBW) * sizeof(float)));
-            tma_load_3d(slot + kOneFaces, &maps.ax, my[q].k0, my[q].j0, my[q].i0, mb);
-            tma_load_3d(slot + kOneFaces + kBX, &maps.ayc, my[q].k0, my[q].j0, my[q].i0, mb);
-            tma_load_3d(slot + kOneFaces + kBX + kBY, &maps.azc, my[q].k0, my[q].j0, my[q].i0, mb);
-        }
-    }
-    wait_boxes();
-    if (!grid_barrier(bar, epoch, ws.err, gridDim.x)) goto finish;
-    {
-        double tot[3];
-        const int comp[3] = {0, 1, 2};
-        scene_sums<3>(bufB, cb, ce, comp, tot, red, ws.tiles);
-        if (threadIdx.x == 0) {
-            init_scalars(Ls, S, false, tot, N);
-            Ls.mean = (double)mean;
-        }
-        __syncthreads();
-    }
-    if (!Ls.live) goto writeback;
-    // ------------------------------------------------------------------------------------------ iterations
-    // k = 0 forms A p0 from the published p0; k >= 1 first advances x, r and p with the scalars of iteration k - 1
-    for (k = 0;; ++k) {
-        const int prev = (k & 1) ^ 1;
-        // k = 0: the p0 boxes (TMA), requested before the scene sums; after that the boxes stay in shared memory and
-        // every block advances its own copy of p at its tiles' cells and face neighbours
-        if (k == 0 && lt == 0) {
-            asm volatile("fence.proxy.async.global;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-#pragma unroll
-            for (int q = 0; q < MAXC; ++q) {
-                if (!have[q]) continue;
-                unsigned long long* mb = &mbar[g * MAXC + q];
-                mbar_expect_tx(mb, (unsigned)(kBZ * sizeof(float)));
-                tma_load_3d(slot_of(q), &maps.p0, my[q].k0 - 4, my[q].j0 - 1, my[q].i0 - 1, mb);
-            }
-        }
-        // k >= 1: the loads of this iteration's scene sums first, then the neighbours' z', q (cp.async), in flight
-        // while the sums are formed
-        double sv[kOneComps][2];
-        if (k > 0) {
-            if (groups >= 2)
-                unit_loads<kOneComps, 2, 2>(prev ? bufB : bufA, units, sv);
-            else
-                unit_loads<kOneComps, 1, 2>(prev ? bufB : bufA, units, sv);
-        }
-        if (k > 0) {
-            const float* Zp = prev ? S.cg_z : S.cg_r;
-            const float* Qp = prev ? S.hdiag : S.cg_Ap;
-            const unsigned hmask = hmask_s[threadIdx.x];
-#pragma unroll
-            for (int q = 0; q < MAXC; ++q) {
-                float* stg = slot_of(q) + kOneHalo;
-                const int tb = (my[q].i0 * n + my[q].j0) * n + my[q].k0;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    int bi = 0, bj = 0, bk = 0;
-                    if (!((hmask >> (4 * q + u)) & 1u)) continue;
-                    halo_point(lt, u, bi, bj, bk);
-                    const int t = tb + (bi * n + bj) * n + bk;
-                    cp_async4(stg + u * 256 + lt, Zp + t);
-                    cp_async4(stg + kOneHaloPts + u * 256 + lt, Qp + t);
-                }
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        }
-        float alpha = 0.0f, beta = 0.0f;
-        bool live = true;   // k = 0 runs only when the set-up left the scene live
-        if (k > 0) {
-            double tot[kOneComps];
-            // pAp, rr, rz, Ap.z, Ap.D.Ap of iteration k - 1: the groups' partials in group order, in every thread
-            if (groups >= 2)
-                unit_sums<kOneComps, 2, 2>(prev ? bufB : bufA, units, sv, tot, red);
-            else
-                unit_sums<kOneComps, 1, 2>(prev ? bufB : bufA, units, sv, tot, red);
-            // every thread derives the same test and scalars from the same sums (no broadcast through shared memory):
-            // the classic test on r_{k-1} (formed in iteration k - 1); converged -> x_{k-1} is the solution
-            const double pAp = tot[0], rr = tot[1], rz = tot[2];
-            const bool above = rr > Ls.atol_sq;
-            live = above && isfinite(rr) && (k - 1) < Ls.maxit;
-            if (live) {
-                const double a = rz / pAp;
-                const double rz_next = rz - 2.0 * a * tot[3] + a * a * tot[4];
-                alpha = __double2float_rn(a);
-                beta = __double2float_rn(rz_next / rz);
-            }
-            if (threadIdx.x == 0) {
-                Ls.iters = k - 1;
-                Ls.rr = rr;
-                Ls.rz = rz;
-                Ls.pAp = pAp;
-                if (!isfinite(rr)) Ls.status |= HF_SCENE_NONFINITE;
-                if (!live && above && isfinite(rr)) Ls.status |= HF_SCENE_PRESSURE_MAXITER;
-                Ls.live = live;
-                Ls.alpha = alpha;
-                Ls.beta = beta;
-            }
-        }
-        if (k == 0) wait_boxes();
-        if (k > 0) asm volatile("cp.async.wait_all;" ::: "memory");
-        asm volatile("bar.sync %0, 256;" ::"r"(g + 1) : "memory");
-        if (!live) break;
-        if (k > 0) {
-            // p_k everywhere in the boxes by one formula: z = z' - alpha q, p = z + beta p_{k-1}; own cells also
-            // advance x and r
-            const unsigned hmask = hmask_s[threadIdx.x];
-#pragma unroll
-            for (int q = 0; q < MAXC; ++q) {
-                float* box = slot_of(q);
-                const float* stg = box + kOneHalo;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    int bi = 0, bj = 0, bk = 0;
-                    if (!((hmask >> (4 * q + u)) & 1u)) continue;
-                    halo_point(lt, u, bi, bj, bk);
-                    float& pb = box[(bi + 1) * 400 + (bj + 1) * 40 + (bk + 4)];
-                    const float z = __fsub_rn(stg[u * 256 + lt], __fmul_rn(alpha, stg[kOneHaloPts + u * 256 + lt]));
-                    pb = __fadd_rn(z, __fmul_rn(beta, pb));
-                }
-                float* X = box + kOneCells;
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const int s = q * 4 + m, e = m * 256 + lt;
-                    const Cell cl = tile_cell(my[q], n, lt, m);
-                    if (!have[q] || !cl.ok) continue;
-                    float& pb = box[(m + 1) * 400 + ((lt >> 5) + 1) * 40 + ((lt & 31) + 4)];
-                    const float zp = __fmul_rn(dg[s], r[s]), qv = __fmul_rn(dg[s], ap[s]);
-                    const float z = __fsub_rn(zp, __fmul_rn(alpha, qv));
-                    X[e] = __fadd_rn(X[e], __fmul_rn(alpha, pb));
-                    r[s] = __fsub_rn(r[s], __fmul_rn(alpha, ap[s]));
-                    pb = __fadd_rn(z, __fmul_rn(beta, pb));
-                }
-            }
-            asm volatile("bar.sync %0, 256;" ::"r"(g + 1) : "memory");
-        }
-        // A p_k from the box; partials of iteration k; publish z_k' = D r_k and q_k = D A p_k
-        {
-            const int cur = k & 1;
-            float* const Zc = cur ? S.cg_z : S.cg_r;
-            float* const Qc = cur ? S.hdiag : S.cg_Ap;
-            __syncthreads();   // red is free (the scene sums above read it)
-            // the five partials of the thread's cells, in cell order (tile q, then m)
-            double part[kOneComps] = {0.0, 0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-            for (int q = 0; q < MAXC; ++q) {
-                const float* slot = slot_of(q);
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const int s = q * 4 + m;
-                    const Cell cl = tile_cell(my[q], n, lt, m);
-                    if (!have[q] || !cl.ok) continue;
-                    const int bj = lt >> 5, bk = lt & 31, o = (m + 1) * 400 + (bj + 1) * 40 + (bk + 4);
-                    const float pk = slot[o];
-                    ap[s] = lap_box(slot, slot + kOneFaces, slot + kOneFaces + kBX, slot + kOneFaces + kBX + kBY, cl, n,
-                                    m, bj, bk, o, hhd);
-                    const float zp = __fmul_rn(dg[s], r[s]);
-                    const double d = dg[s], a = ap[s], rs = r[s], z = zp;
-                    part[0] += (double)pk * a;
-                    part[1] += rs * rs;
-                    part[2] += rs * z;
-                    part[3] += a * z;
-                    part[4] += a * (d * a);
-                    // only cells on the tile's faces are another tile's face neighbours
-                    if (m == 0 || m == 3 || bj == 0 || bj == 7 || bk == 0 || bk == 31) {
-                        Zc[cl.t] = zp;
-                        Qc[cl.t] = __fmul_rn(dg[s], ap[s]);
-                    }
-                }
-            }
-            stash_warp<kOneComps>(part, red, 0);
-            publish_unit<kOneComps>(red, cur ? bufB : bufA, unit, units);
-        }
-        if (!grid_barrier(bar, epoch, ws.err, gridDim.x)) goto finish;
-    }
-writeback:
-    // -------------------------------------------------- write x back, then project the faces
-#pragma unroll
-    for (int q = 0; q < MAXC; ++q) {
-        const float* X = slot_of(q) + kOneCells;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const Cell cl = tile_cell(my[q], n, lt, m);
-            if (have[q] && cl.ok) xg[cl.t] = X[m * 256 + lt];
-        }
-    }
-    if (!grid_barrier(bar, epoch, ws.err, gridDim.x)) goto finish;
-    {
-        const float dtr = (float)(dt_d / S.rho);
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q) {
-            const float* X = slot_of(q) + kOneCells;
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const Cell cl = tile_cell(my[q], n, lt, m);
-                if (have[q] && cl.ok)
-                    project_cell(S, S.u[par ^ 1], S.v[par ^ 1], S.w[par ^ 1], S.p, X[m * 256 + lt], dtr, h, cl);
-            }
-        }
-    }
-finish:
-    if (*(volatile int*)ws.err) {
-        // leave no copy in flight: the last requested boxes are waited for again (bounded) before the block exits
-#pragma unroll
-        for (int q = 0; q < MAXC; ++q)
-            if (have[q]) mbar_wait(&mbar[g * MAXC + q], phase_bit ^ 1u);
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    if (blockIdx.x == 0 && threadIdx.x == 0) write_stats(S, Ls, false, *(volatile int*)ws.err != 0, par);
-}
-
-const void* pcg_one_kernel(int maxc) {
-    if (maxc == 1) return (const void*)k_pcg_one<1>;
-    if (maxc == 2) return (const void*)k_pcg_one<2>;
-    return (const void*)k_pcg_one<3>;
-}
-
-size_t pcg_one_smem(int groups, int maxc) { return (size_t)groups * maxc * kOneSlotFloats * sizeof(float) + 128; }
 
 const void* pcg_kernel(bool heat, bool tma) {
     return heat ? (const void*)k_pcg<true, false> : tma ? (const void*)k_pcg<false, true> : (const void*)k_pcg<false, false>;

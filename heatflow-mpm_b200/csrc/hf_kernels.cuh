@@ -29,7 +29,7 @@ struct Workspace {
     const CUtensorMap* maps;  // [kMapsPerScene S] per scene: the stencil boxes z, p_0, p_1, alpha_f x, alpha_f y (cells),
                               // alpha_f z (cells); then tile boxes of x (p), p_0, p_1, r, Ap, D
     double* partA;          // [3 T] per-tile fp64 partials of CG phase A, component-major: component c of tile t at
-                            // c * tiles + t (the single-reduction kernel: 5 components per 256-thread group)
+                            // c * tiles + t
     double* partB;          // [3 T] per-tile fp64 partials of the CG set-up and phase B (same layout)
     double* mean_part;      // [C] per-chunk fp64 sums of the pressure rhs
     // the on-chip pressure solve (hf_brick.cu); absent from the workspace of a plan that only streams
@@ -59,12 +59,6 @@ int brick_box_bytes();
 int brick_set_wait_limit(unsigned long long limit_ns, int absent_block);
 // workspace bytes of a plan without the on-chip solve's part (streaming plans)
 size_t streaming_workspace_bytes(int num_scenes, int num_chunks, int num_tiles);
-
-// TMA descriptors of the tiled pressure stencil (resident CG): z, both search-direction buffers, alpha_f x (the u
-// lattice), and the cell-layout copies of alpha_f y and z.
-struct TileMaps {
-    CUtensorMap z, p0, p1, ax, ayc, azc;
-};
 
 __global__ void k_scatter(const hf_scene* __restrict__ scenes, int s);
 __global__ void k_obstacle(const hf_scene* __restrict__ scenes, const WorkItem* __restrict__ work, int all_scenes);
@@ -96,11 +90,6 @@ __global__ void k_heat_matvec_plain(int n, float h, float dt, float alpha, float
 const void* pcg_kernel(bool heat, bool tma);
 // dynamic shared memory of the streaming kernel (tma: one stencil slot per block, staged with TMA)
 size_t pcg_stream_smem(bool tma);
-// single-reduction register-resident pressure solve of one scene with n % 4 == 0 (one grid barrier per CG iteration;
-// uses hdiag as scratch), the same arguments and thread layout as the TMA resident variant; dynamic shared memory
-// pcg_one_smem(groups, maxc)
-const void* pcg_one_kernel(int maxc);
-size_t pcg_one_smem(int groups, int maxc);
 // limit of the CG kernels' bounded waits on the current device and the block kept from the first grid barrier
 // (-1: none); synchronous (constant memory)
 int set_wait_limit(unsigned long long limit_ns, int absent_block);

@@ -286,7 +286,7 @@ class ScenePlan:
 
     @property
     def resident_tiles(self):
-        """Tiles per 256-thread group of the single-scene resident CG variant (0: the fewest that fit)."""
+        """Accepted (0..3), without effect: the on-chip CG solves choose their tiles per block from the scenes."""
         return (self.plan.options >> _lib.HF_PLAN_RES_TILES_SHIFT) & 3
 
     @resident_tiles.setter
@@ -297,9 +297,8 @@ class ScenePlan:
 
     @property
     def single_reduction_cg(self):
-        """Pressure solve of a single-scene plan (n % 4 == 0) with one grid barrier per CG iteration: the classic
-        vector recurrences, beta from the expansion of the next r.z in the iteration's partials, the classic stopping
-        test; results within ~1e-6 relative of the classic method.  Off by default."""
+        """Asks for a pressure solve within ~1e-6 relative of the classic method.  The on-chip classic solve serves it:
+        its iteration takes less time than one with a single reduction point did."""
         return bool(self.plan.options & _lib.HF_PLAN_SINGLE_REDUCTION_CG)
 
     @single_reduction_cg.setter

@@ -5,9 +5,8 @@ Same constructor, methods and attributes as the reference.  One extra keyword, `
 and velocities; used when Newton is not installed) or a body object of the caller's (``mpm.DLPackBody`` interface).  The air substep itself -- obstacle fields, temperature stages,
 heat CG, FLIP particle update, face stage, pressure CG and projection -- is one call into libheatflow_b200, replayed
 from a CUDA graph after the first substep at each dt (``graph=False``: launched directly every time; same bits).
-``cg="single-reduction"`` solves the pressure system with one grid barrier per CG iteration instead of two (the classic
-recurrences with beta from an expansion of the next r.z; the same stopping test; results within ~1e-6 relative of the
-classic method, which stays the default)."""
+``cg="single-reduction"`` allows a pressure solve within ~1e-6 relative of the classic method, the default; the on-chip
+classic solve serves both (8.2 us an iteration at 96^3; a kernel with one reduction point per iteration took 10.3)."""
 from __future__ import annotations
 
 from dataclasses import asdict

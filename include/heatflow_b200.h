@@ -118,23 +118,20 @@ typedef struct hf_scene {
 } hf_scene;
 
 /* hf_plan.options */
-#define HF_PLAN_STREAMING_CG 1u      /* never use the register-resident CG variant (single-scene plans use it when
-                                        the scene's tiles fit one block per SM) */
-#define HF_PLAN_NO_TMA 2u            /* resident pressure CG without the TMA-staged stencil */
+#define HF_PLAN_STREAMING_CG 1u      /* never use the on-chip CG solves (plans use them when every active scene fits: edges
+                                        up to 168) */
+#define HF_PLAN_NO_TMA 2u            /* the streaming pressure CG without the TMA-staged stencil */
 #define HF_PLAN_STREAMING_HEAT 4u    /* the heat CG of a single-scene plan in the streaming kernel (pressure unchanged) */
-#define HF_PLAN_SINGLE_REDUCTION_CG 8u /* single-scene plans with n % 4 == 0: the pressure solve with one grid barrier
-                                          per CG iteration instead of two -- the classic vector recurrences, beta from
-                                          the expansion of the next r.z in the iteration's partials (D'Azevedo,
-                                          Eijkhout & Romine 1993), the classic stopping test; results within ~1e-6
-                                          relative of the classic method, so it is off by default.  Uses the scene's
-                                          hdiag as scratch during the pressure solve. */
+#define HF_PLAN_SINGLE_REDUCTION_CG 8u /* accepted for a pressure solve within ~1e-6 relative of the classic method; served
+                                          by the on-chip classic solve, whose iteration takes less time than one with
+                                          a single reduction point did (8.2 against 10.3 us at 96^3) */
 #define HF_PLAN_MAPS_READY 0x8000u   /* set by hf_plan_upload: the workspace holds the scenes' TMA descriptors (the
                                         streaming pressure CG stages its stencil boxes with TMA when every active scene
                                         has n % 4 == 0) */
 #define HF_PLAN_LANES_SHIFT 8        /* options bits 8..11: lanes of the streaming CG launch (independent scene groups
                                         solved side by side, each lane with its own barrier; 0 = one lane) */
-#define HF_PLAN_RES_TILES_SHIFT 12   /* options bits 12..13: tiles per 256-thread group of the resident CG variant (1..3;
-                                        0 = the fewest that fit; more tiles per group = fewer threads, more registers) */
+#define HF_PLAN_RES_TILES_SHIFT 12   /* options bits 12..13: accepted, without effect (the on-chip solves choose their tiles per
+                                        block from the scenes) */
 
 /* A batch of scenes ready to launch: tables in device memory plus the host copy used to size launches. */
 typedef struct hf_plan {
