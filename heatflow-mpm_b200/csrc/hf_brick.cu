@@ -2,14 +2,17 @@
 //
 // Same systems, arithmetic and reduction trees as the streaming kernel (hf_cg.cu): the pressure solve -- mean removal,
 // Jacobi-preconditioned CG warm-started from p, projection, end of the substep (grid.py:235-251, 94-153) -- and the heat
-// solve (heat.py:198-210).  A team of blocks (one per SM) owns a scene's tiles in contiguous runs of whole units; r, A p (and D) of a block's cells live in registers, p
-// and x in shared memory, so an iteration moves only what blocks owe each other.  A plan of several scenes gives every
-// scene a team of its own and a place in the blocks' common order (BrickJobs, hf_api.cu); teams work side by side.
+// solve (heat.py:198-210).  A team of blocks (one per SM) owns a scene's tiles in contiguous runs of whole units; r, A p
+// (and D) of a block's cells live in registers, p and x in shared memory, so an iteration moves only what blocks owe each
+// other.  A plan of several scenes gives every scene a team of its own and a place in the blocks' common order
+// (brick_schedule, hf_api.cu); teams work side by side.
 //
-// What bounds an iteration is latency: two reductions of the whole scene (p.Ap; r.r and r.z) and one halo exchange.  A
-// barrier followed by reading the partials costs a release, an atomic, an acquire poll and another round trip (3450 + 2300
-// cycles for 148 blocks of 512 threads).  Here every value carries its own arrival mark instead, so no fence, counter or
-// barrier is involved and one trip through L2 does:
+// What bounds an iteration: two reductions of the whole scene (p.Ap; r.r and r.z), one halo exchange, and between them the
+// issue of some 90 instructions per cell (96^3: 16,300 cycles, of which 7,800 for the exchanges; 45 % issue).  A barrier
+// followed by reading the partials costs a release, an atomic, an acquire poll and another round trip (3450 + 2300 cycles
+// for 148 blocks of 512 threads).  Here every value carries its own arrival mark instead, so no fence, counter or barrier
+// is involved and one trip through L2 does.  Microseconds per pressure iteration, the kernels before -> this one: 32^3
+// 6.6 -> 4.6, 75^3 15.8 -> 7.3, 96^3 13.5 -> 8.2, 128^3 33.8 -> 19.8, 160^3 69.2 -> 35.3.
 //   * reductions: a block adds its tiles' partials into unit sums and posts each on a 128-byte line of its own as {low
 //     word, tag, high word, tag}, self-validating 8-byte halves; every member polls all lines of its team.  A line that
 //     is being polled takes one store, of one warp instruction: measured alone, 148 blocks and two values, 1830 to 2400
@@ -429,8 +432,11 @@ __global__ void __launch_bounds__(256 * G, 1)
         float ahead[kRowsEach];
         auto await = [&](int r, unsigned tag, unsigned long long v) {
             const unsigned long long* from = ws.halo + rows[r].x + lane;
+            // A neighbour whose last sums told it that the solve has ended may already have put x in z's place.  That is as
+            // good as z here: this block is about to learn the same, and z is not used any more.
+            const unsigned after = team.base | ((tag + 1) & 0x3ffu);
             Patience patience;
-            while (__any_sync(0xffffffffu, (unsigned)(v >> 32) != tag)) {   // the warp stays together
+            while (__any_sync(0xffffffffu, (unsigned)(v >> 32) != tag && (unsigned)(v >> 32) != after)) {   // together
                 if (__any_sync(0xffffffffu, !patience.more(err))) {
                     bad = 1;
                     break;
