@@ -23,7 +23,7 @@ import torch
 
 from . import _lib
 from .heater import FAN, K_SOLID, BoxHeater, Heater, face_masks, fan_momentum, source_rate
-from .scene import DeviceScene, SceneSpec, ScenePlan
+from .scene import DeviceScene, SceneSpec, ScenePlan, recording
 from .solver import wall_fixed
 from .voxelize import device_statics, sphere_bounds
 
@@ -176,7 +176,7 @@ class AirBatch:
             self.plan.substep(dt)
         torch.cuda.current_stream(self.device).wait_stream(s)
         g = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(g, stream=s):
+        with recording(g, s):
             for _ in range(k):
                 self.plan.substep(dt)
         self.graph, self._graph_key = g, key

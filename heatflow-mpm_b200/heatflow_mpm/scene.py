@@ -11,6 +11,9 @@ the static face weights, alpha_s at the static solid fraction) and the particle 
 from __future__ import annotations
 
 import ctypes as C
+import gc
+import threading
+from contextlib import contextmanager
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -238,6 +241,32 @@ class DeviceScene:
 
     def set_current(self, name, value):
         self.current(name).copy_(torch.as_tensor(np.asarray(value, np.float32), device=self.device))
+
+
+_recording = threading.Lock()   # one recording at a time: each restores the collector's state as it found it
+
+
+@contextmanager
+def recording(graph, stream):
+    """Record what is launched on `stream` into `graph` (thread-local mode: a frame writer's thread may wait on its own
+    copies meanwhile).  torch.cuda.graph would also collect garbage and give all cached memory back to the driver -- from
+    tens of milliseconds to over a second -- which a recording that allocates nothing does not need; it must only not be
+    interrupted by a collection that frees CUDA objects.  A graph that this one replaces is no longer in flight: the
+    device is synchronised first."""
+    torch.cuda.synchronize(stream.device)
+    with _recording:
+        collecting = gc.isenabled()
+        gc.disable()
+        try:
+            with torch.cuda.stream(stream):
+                graph.capture_begin(capture_error_mode="thread_local")
+                try:
+                    yield
+                finally:
+                    graph.capture_end()
+        finally:
+            if collecting:
+                gc.enable()
 
 
 class ScenePlan:

@@ -19,7 +19,7 @@ from .grid import AirGrid, GridConfig, grid_edge
 from .heat import HeatField
 from .heater import Heater
 from .mpm import FrozenBody, Material, ThermalMPM
-from .scene import DeviceScene, SceneSpec, ScenePlan
+from .scene import DeviceScene, SceneSpec, ScenePlan, recording
 
 KAPPA_AIR = 2.2e-5     # solver.py:15
 K_PARTICLE = 1.0e-3    # solver.py:16
@@ -138,8 +138,7 @@ class HeatflowMPM:
         side = torch.cuda.Stream(dev)
         side.wait_stream(cur)
         g = torch.cuda.CUDAGraph()
-        # thread-local capture: a frame writer's thread may wait on its own copies meanwhile
-        with torch.cuda.graph(g, stream=side, capture_error_mode="thread_local"):
+        with recording(g, side):
             plan.substep(dt)
         cur.wait_stream(side)
         self._graph, self._graph_key = g, key
