@@ -20,8 +20,10 @@
 //   * halo: z of the cells on faces that a tile shares with another block's tile, as {z, tag} words that the neighbour
 //     polls (again one store for each run of 32).  Each block advances its own copy of p there by the owner's operations
 //     on the owner's values.
-// Tags name launch, job and step, so nothing has to be cleared between launches.  A line alternates with the parity of
-// the step: a member posts step s + 2 only after step s + 1, which every member posted after reading step s.
+// Tags name launch (12 bits), job and step (10 bits each), so nothing has to be cleared between launches: every launch
+// rewrites each word that its members poll -- a unit's two lines at step 1, the shared faces at the set-up -- so a tag of
+// 4096 launches ago is never still there.  A line alternates with the parity of the step: a member posts step s + 2 only
+// after step s + 1, which every member posted after reading step s.
 #include "hf_cg.cuh"
 
 namespace hf {
@@ -195,6 +197,9 @@ __device__ __forceinline__ bool exchange(const Team& team, int nt, unsigned& ste
                 for (int q = 0; q < kAtOnce; ++q) s += v[q];
             }
             st_halves(team.post + ((step & 1u) * kLines + u) * 8 + c, s, tag);
+            // The line of the even steps as well, under a tag that nobody looks for there: a solve may end before its first
+            // even step, and what an older launch left would come up again when the launch number has gone round.
+            if (step == 1) st_halves(team.post + u * 8 + c, s, tag);
         }
     }
     if (warp >= kPollWarps) {

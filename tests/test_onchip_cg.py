@@ -56,3 +56,53 @@ def test_batch_equals_streaming(sizes):
             plan.substep(2e-3)
     for a, b in zip(chip, stream):
         _equal(a, b)
+
+
+def test_launch_number_wraps():
+    """The tags keep 12 bits of the launch number.  A heat solve of one iteration, solves of none up to the wrap, then one
+    that iterates again from another state, with the first one's tags: it equals the streaming kernel's, bit for bit (no
+    block takes a sum that the first launch left behind)."""
+    import torch
+    from heatflow_mpm.scene import ScenePlan
+    dt = 2e-3
+    (a,), (b,) = _scenes([24], 60), _scenes([24], 60)
+    chip, stream = ScenePlan([a]), ScenePlan([b], streaming_cg=True)
+    rng = np.random.default_rng(4)
+    first, last = ((25.0 + rng.uniform(-c, c, (24, 24, 24))).astype(np.float32) for c in (2.0, 9.0))
+    for plan, sc in ((chip, a), (stream, b)):
+        plan.prepare_statics()
+        nxt = sc.T[sc.parity() ^ 1]
+        for start in (first, last):
+            nxt.copy_(torch.as_tensor(start))
+            sc.hrhs.copy_(torch.as_tensor(start))
+            plan.heat_solve(dt)
+            iters = sc.read_state().heat_iters
+            assert iters == 1 if start is first else iters >= 1
+            if start is first and plan is chip:
+                for _ in range(4095):
+                    plan.heat_solve(dt)
+                assert sc.read_state().heat_iters == 0
+        sc.result = nxt.cpu().numpy()
+    assert np.array_equal(a.result, b.result)
+    assert a.read_state().heat_rr == b.read_state().heat_rr and a.read_state().status == 0
+
+
+def test_step_numbers_wrap():
+    """The tags keep 10 bits of the step: more than 1024 iterations (two steps and one halo exchange each), forced by face
+    fractions over six decades."""
+    import torch
+    from heatflow_mpm.scene import ScenePlan
+    (a,), (b,) = _scenes([32], 60), _scenes([32], 60)
+    for sc in (a, b):
+        sc.spec.cg_max_iter, sc.spec.cg_tol = 1200, 1e-30
+    rng = np.random.default_rng(6)
+    weights = [torch.as_tensor((10.0 ** rng.uniform(-6, 0, s.shape)).astype(np.float32)) for s in (a.ax, a.ay, a.az)]
+    for sc, plan in ((a, ScenePlan([a])), (b, ScenePlan([b], streaming_cg=True))):
+        plan.prepare_statics()
+        for dst, w in zip((sc.ax, sc.ay, sc.az), weights):
+            dst.copy_(w)
+        for dst, w in ((sc.ayc, sc.ay[:, :-1]), (sc.azc, sc.az[:, :, :-1])):
+            dst.copy_(w)
+        plan.substep(2e-3)
+    assert a.read_state().pressure_iters == 1200
+    _equal(a, b)
