@@ -143,6 +143,25 @@ __device__ __forceinline__ void div_rn4(float (&x)[4], const DivBy& d) {
     }
 }
 
+// a job's word in ws.arrive: members that are done with it; a member gave up, and the scene's parity that it started from
+constexpr unsigned kArrived = 0xffffu, kGaveUp = 1u << 30, kParity = 1u << 31;
+
+// The scenes of a launch of which any member gave up are timeouts, whatever their first blocks found: not counted, old parity.
+// (A function of its own: in line, its registers made an iteration at 96^3 5 % slower.)
+__device__ __noinline__ void take_back(const hf_scene* scenes, const unsigned* arrive, const int4* of, int jobs, int only, bool heat) {
+    __threadfence();
+    for (int q = 0; q < jobs; ++q) {
+        const unsigned a = *(volatile const unsigned*)(arrive + q);
+        if (!(a & kGaveUp)) continue;
+        volatile hf_scene_state* st = scenes[jobs == 1 ? only : of[q].x].state;
+        st->status |= HF_SCENE_BARRIER_TIMEOUT;
+        if (!heat && st->parity != (int)(a / kParity)) {
+            st->parity ^= 1;
+            st->substeps -= 1;
+        }
+    }
+}
+
 // A block's place in a team.  A block owns at most as many units as tiles.
 constexpr int kLines = kBrickWideTiles;        // lines of a block and parity
 struct Team {
@@ -279,7 +298,8 @@ __global__ void __launch_bounds__(256 * G, 1)
     __shared__ LocalScene Ls;
     __shared__ hf_scene Ss;
     __shared__ float dtab[8];
-    __shared__ int s_count[5];                    // i planes, j slots, k columns, rows, face boxes in use
+    __shared__ int s_count[6];                    // i planes, j slots, k columns, rows, face boxes in use; [5]: s_gave_up
+    int& s_gave_up = s_count[5];                  // a job of this block did not end for a wait that gave up (thread 0)
     const int g = threadIdx.x >> 8, lt = threadIdx.x & 255, lane = lt & 31, row = lt >> 5, warp = threadIdx.x >> 5;
     int* const err = reinterpret_cast<int*>(ws.brick + 2);
     const unsigned launch = *(volatile unsigned*)ws.brick;
@@ -287,6 +307,7 @@ __global__ void __launch_bounds__(256 * G, 1)
     const int pages = bl.tiles * (kWide ? 1024 : 2048), boxes = pages + bl.pages * 1024;
     int bad = 0;                                  // a wait of this thread gave up
     int left = -1, left_nb = 0;                   // the job before and its blocks
+    if (threadIdx.x == 0) s_gave_up = 0;
 
     for (int job = 0; job < bl.jobs; ++job) {
         const int4 J = bl.jobs == 1 ? bl.job0 : ws.jobs[job];   // scene, first block, blocks
@@ -378,7 +399,7 @@ __global__ void __launch_bounds__(256 * G, 1)
         if (left >= 0 && threadIdx.x == 0) {
             // everyone has read this block's last sums of the job before: its lines may be written again
             Patience patience;
-            while (ld_acquire_u32(ws.arrive + left) < (unsigned)left_nb)
+            while ((ld_acquire_u32(ws.arrive + left) & kArrived) < (unsigned)left_nb)
                 if (!patience.more(err)) {
                     bad = 1;
                     break;
@@ -929,7 +950,7 @@ __global__ void __launch_bounds__(256 * G, 1)
                     if (kWide) x = m < cells ? S.p[t + m * nn] : 0.0f;
                     x4[m] = x;
                 }
-                post(tt[q], x4, team.base | (pub & 0x3ffu));
+                if ((int)blockIdx.x != c_absent_block - kAbsentLate) post(tt[q], x4, team.base | (pub & 0x3ffu));
             }
             __syncthreads();
             if (warp >= kPollWarps) fetch(team.base | (pub & 0x3ffu));
@@ -983,6 +1004,14 @@ __global__ void __launch_bounds__(256 * G, 1)
             }
         }
         __syncthreads();
+        if (!ok) {
+            // The first block reports the scene, and it may have finished where this one gave up: the last block to leave the
+            // launch then takes that back (below).
+            if (threadIdx.x == 0) {
+                s_gave_up = 1;
+                atomicOr(ws.arrive + job, kGaveUp | (par ? kParity : 0u));
+            }
+        }
         if (bl.jobs > 1 && threadIdx.x == 0) {
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ws.arrive + job) : "memory");
             left = job;
@@ -995,8 +1024,11 @@ __global__ void __launch_bounds__(256 * G, 1)
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        if (atomicAdd(ws.brick + 1, 1u) == gridDim.x - 1) {
-            if (bl.jobs > 1)
+        const unsigned before = atomicAdd(ws.brick + 1, s_gave_up ? 0x10001u : 1u);   // low half: blocks; high: those that gave up
+        if ((before & 0xffffu) == gridDim.x - 1) {
+            const bool any = s_gave_up || before >> 16;
+            if (any) take_back(scenes, ws.arrive, ws.jobs, bl.jobs, bl.job0.x, HEAT);
+            if (bl.jobs > 1 || any)
                 for (int q = 0; q < bl.jobs; ++q) ws.arrive[q] = 0;
             ws.brick[1] = 0;
             ws.brick[2] = 0;

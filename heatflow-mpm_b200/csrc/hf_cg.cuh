@@ -7,12 +7,14 @@
 namespace hf {
 
 constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;   // 2 s
-// Limit of every bounded wait of the CG kernels (grid and lane barriers, TMA copies), and the block that does not
-// arrive at the first grid barrier of each persistent CG launch (-1: none).  The defaults are what every solve uses;
-// hf_set_wait_limit changes both, so that a test can make a barrier's wait run out on purpose and check that the
-// kernel reports HF_SCENE_BARRIER_TIMEOUT and returns with the context usable.
+// Limit of every bounded wait of the CG kernels (grid and lane barriers, TMA copies, tagged words), and the block that does
+// not arrive at the first grid barrier (or first exchange) of each persistent CG launch (-1: none; kAbsentLate + b: block b
+// of an on-chip pressure solve keeps its final pressures on shared faces to itself).  The defaults are what every solve
+// uses; hf_set_wait_limit changes both, so that a test can make a wait run out on purpose and check that the kernel reports
+// HF_SCENE_BARRIER_TIMEOUT and returns with the context usable.
 static __constant__ unsigned long long c_wait_limit_ns = kBarrierTimeoutNs;
 static __constant__ int c_absent_block = -1;
+constexpr int kAbsentLate = 65536;
 
 __device__ __forceinline__ int uidx_(int n, int i, int j, int k) { return (i * n + j) * n + k; }
 __device__ __forceinline__ int vidx_(int n, int i, int j, int k) { return (i * (n + 1) + j) * n + k; }

@@ -34,7 +34,7 @@ struct Workspace {
     double* mean_part;      // [C] per-chunk fp64 sums of the pressure rhs
     // the on-chip pressure solve (hf_brick.cu); absent from the workspace of a plan that only streams
     unsigned* brick;        // launches so far, blocks that have left this launch, a wait of this launch gave up
-    unsigned* arrive;       // [S] members that have left a job
+    unsigned* arrive;       // [S] members that have left a job; a member gave up (kGaveUp, hf_brick.cu)
     int4* jobs;             // [S] (scene, first block, blocks) in the blocks' common order
     ulonglong2* mail;       // [blocks][2][kBrickWideTiles] 128-byte lines: every block's unit sums, two steps deep
     unsigned long long* halo;   // [kHaloEntries T] (value, tag) words of the tiles' faces

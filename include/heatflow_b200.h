@@ -222,8 +222,9 @@ int hf_k_divide_by(int count, const float *x, float y, float *out, void *stream)
    CG kernels -- grid and lane barriers, TMA copies -- gives up after limit_ns (default 2 s), sets
    HF_SCENE_BARRIER_TIMEOUT in the scenes of the launch, and every block returns, leaving the context usable.
    absent_block >= 0 keeps that block of each CG launch from arriving at its first grid barrier, so that a test can
-   make the wait run out on purpose (-1: normal operation).  Applies to later launches on the current device;
-   synchronous.  Restore (2000000000, -1) after a test. */
+   make the wait run out on purpose (-1: normal operation); absent_block >= 65536 lets block absent_block - 65536
+   of an on-chip pressure solve keep its final pressures from its neighbours, whose last wait then runs out.  Applies to later
+   launches on the current device; synchronous.  Restore (2000000000, -1) after a test. */
 int hf_set_wait_limit(unsigned long long limit_ns, int absent_block);
 
 /* ------------------------------------------------------------------------------------ scene set-up on the device */

@@ -129,3 +129,28 @@ def test_barrier_timeout_is_reported_and_the_device_stays_usable(torch_cuda, var
     st2 = sc2.read_state()
     assert st2.status == 0 and st2.substeps == 1
     assert np.isfinite(sc2.current("T").cpu().numpy()).all()
+
+
+def test_timeout_of_one_block_at_the_end_is_reported(torch_cuda):
+    """The last block of an on-chip pressure solve keeps its final pressures from its neighbours, whose waits run out after
+    every sum was exchanged; the first block, which has no such neighbour, finishes.  The scene's status says so all the
+    same (one tile a block, and two), the substep is not counted and the parity stays; the next substep runs normally."""
+    torch = torch_cuda
+    from heatflow_mpm import _lib
+    L = _lib.load()
+    for n, blocks in ((32, 32), (64, 148)):
+        sc, plan = _plain(n)
+        torch.cuda.synchronize()
+        _lib.check(L.hf_set_wait_limit(1_000_000, 65536 + blocks - 1), "hf_set_wait_limit")
+        try:
+            plan.substep(DT)
+            torch.cuda.synchronize()
+        finally:
+            _lib.check(L.hf_set_wait_limit(_lib.WAIT_LIMIT_NS, -1), "hf_set_wait_limit")
+        st = sc.read_state()
+        assert st.status & _lib.HF_SCENE_BARRIER_TIMEOUT, (n, st.status)
+        assert st.parity == 0 and st.substeps == 0, n
+        sc.p.zero_()
+        plan.substep(DT)
+        st = sc.read_state()
+        assert st.status == 0 and st.substeps == 1 and st.parity == 1, n
