@@ -69,18 +69,27 @@ __device__ __forceinline__ ulonglong2 ld_halves(const ulonglong2* p) {
     return v;
 }
 
+// The limit of a wait has passed.  At a job's start others may still be busy with an earlier job: as long as any team of the
+// launch has finished an iteration since t0 (its first block notes the time beside err), the wait begins anew from there.
+__device__ __forceinline__ unsigned long long extend(int* err, unsigned long long t0, bool start) {
+    const unsigned long long beat = ld_relaxed(reinterpret_cast<unsigned long long*>(err + 2));
+    if (start && (long long)(beat - t0) > 0) return beat;
+    atomicExch(err, 1);
+    return 0;
+}
+
 // A bounded wait's clock: false once the limit has passed or another block has given up (which sets err).
 struct Patience {
     unsigned long long t0 = 0;
     unsigned spins = 0;
-    __device__ __forceinline__ bool more(int* err) {
+    __device__ __forceinline__ bool more(int* err, bool start) {
         if (++spins & 63u) return true;
         if (*(volatile int*)err) return false;
         const unsigned long long now = global_timer_ns();
         if (!t0) t0 = now;
-        if (now - t0 <= c_wait_limit_ns) return true;
-        atomicExch(err, 1);
-        return false;
+        if ((long long)(now - t0) <= (long long)c_wait_limit_ns) return true;
+        t0 = extend(err, t0, start);
+        return t0 != 0;
     }
 };
 
@@ -245,7 +254,7 @@ __device__ __forceinline__ bool exchange(const Team& team, int nt, unsigned& ste
                 }
             }
             if (__all_sync(0xffffffffu, here)) break;
-            if (__any_sync(0xffffffffu, !patience.more(team.err))) {
+            if (__any_sync(0xffffffffu, !patience.more(team.err, step == 1))) {
                 bad = 1;
                 break;
             }
@@ -400,7 +409,7 @@ __global__ void __launch_bounds__(256 * G, 1)
             // everyone has read this block's last sums of the job before: its lines may be written again
             Patience patience;
             while ((ld_acquire_u32(ws.arrive + left) & kArrived) < (unsigned)left_nb)
-                if (!patience.more(err)) {
+                if (!patience.more(err, true)) {
                     bad = 1;
                     break;
                 }
@@ -463,7 +472,7 @@ __global__ void __launch_bounds__(256 * G, 1)
             const unsigned after = team.base | ((tag + 1) & 0x3ffu);
             Patience patience;
             while (__any_sync(0xffffffffu, (unsigned)(v >> 32) != tag && (unsigned)(v >> 32) != after)) {   // together
-                if (__any_sync(0xffffffffu, !patience.more(err))) {
+                if (__any_sync(0xffffffffu, !patience.more(err, (tag & 0x3ffu) == 1))) {
                     bad = 1;
                     break;
                 }
@@ -484,6 +493,8 @@ __global__ void __launch_bounds__(256 * G, 1)
                 const int r = warp - kPollWarps + u * kRowWarps;
                 if (r < nrows) ahead[u] = await(r, tag, v[u]);
             }
+            if (bl.jobs > 1 && leader && threadIdx.x == 32 * kPollWarps)   // for who waits for this team's blocks (extend)
+                st_relaxed(reinterpret_cast<unsigned long long*>(ws.brick + 4), global_timer_ns());
         };
         auto take = [&](unsigned tag, auto apply) {
             auto place = [&](int r) {

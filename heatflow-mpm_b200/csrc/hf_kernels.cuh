@@ -33,7 +33,8 @@ struct Workspace {
     double* partB;          // [3 T] per-tile fp64 partials of the CG set-up and phase B (same layout)
     double* mean_part;      // [C] per-chunk fp64 sums of the pressure rhs
     // the on-chip pressure solve (hf_brick.cu); absent from the workspace of a plan that only streams
-    unsigned* brick;        // launches so far, blocks that have left this launch, a wait of this launch gave up
+    unsigned* brick;        // launches so far, blocks that have left this launch, a wait of this launch gave up; at [4], 64
+                            // bits: when a team last finished an iteration
     unsigned* arrive;       // [S] members that have left a job; a member gave up (kGaveUp, hf_brick.cu)
     int4* jobs;             // [S] (scene, first block, blocks) in the blocks' common order
     ulonglong2* mail;       // [blocks][2][kBrickWideTiles] 128-byte lines: every block's unit sums, two steps deep

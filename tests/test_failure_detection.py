@@ -154,3 +154,38 @@ def test_timeout_of_one_block_at_the_end_is_reported(torch_cuda):
         plan.substep(DT)
         st = sc.read_state()
         assert st.status == 0 and st.substeps == 1 and st.parity == 1, n
+
+
+def test_waiting_for_another_scene_is_no_timeout(torch_cuda):
+    """Five scenes that share the on-chip solves' blocks: the fourth starts on blocks of the first two, one of which takes
+    2000 iterations (some 14 ms) and one a few.  With a wait limit of 1 ms the blocks that are there early wait for longer
+    than the limit, but the scene they wait for makes progress: no scene times out."""
+    torch = torch_cuda
+    from heatflow_mpm import _lib
+    from heatflow_mpm.scene import DeviceScene, ScenePlan
+    L = _lib.load()
+    scenes = []
+    for i, (n, tol) in enumerate(((96, 1e-30), (96, 0.5), (80, 1e-4), (72, 1e-4), (24, 1e-4))):
+        spec, T0, uvw = random_scene_inputs(n, seed=20 + i)
+        spec.cg_tol = tol
+        if i == 0:
+            spec.cg_max_iter = 2000
+        sc = DeviceScene(spec)
+        sc.set_current("T", T0)
+        for nm, a in zip("uvw", uvw):
+            sc.set_current(nm, a)
+        scenes.append(sc)
+    plan = ScenePlan(scenes)
+    plan.prepare_statics()
+    torch.cuda.synchronize()
+    _lib.check(L.hf_set_wait_limit(1_000_000, -1), "hf_set_wait_limit")
+    try:
+        plan.substep(DT)
+        torch.cuda.synchronize()
+    finally:
+        _lib.check(L.hf_set_wait_limit(_lib.WAIT_LIMIT_NS, -1), "hf_set_wait_limit")
+    states = [sc.read_state() for sc in scenes]
+    assert states[0].pressure_iters > 1000, states[0].pressure_iters
+    assert not any(st.status & _lib.HF_SCENE_BARRIER_TIMEOUT for st in states), [st.status for st in states]
+    assert [st.status for st in states[1:]] == [0] * 4
+    assert all(st.substeps == 1 for st in states)
