@@ -672,6 +672,14 @@ int hf_k_divide_by(int count, const float* x, float y, float* out, void* stream)
     return HF_OK;
 }
 
+int hf_k_quotient(int count, const double* a, const double* b, double* out, void* stream) {
+    if (count < 0 || (count > 0 && (!a || !b || !out))) return fail(HF_ERR_ARG, "hf_k_quotient: bad arguments");
+    if (count == 0) return HF_OK;
+    hf::k_quotient<<<592, 256, 0, S(stream)>>>(count, a, b, out);
+    HF_CUDA(cudaGetLastError(), "launch (quotient)");
+    return HF_OK;
+}
+
 int hf_k_laplacian(int n, double h, double alpha, double beta, const float* p, const float* ax, const float* ay,
                    const float* az, const float* y, float* out, void* stream) {
     if (n < 1 || !p || !ax || !ay || !az || !y || !out) return fail(HF_ERR_ARG, "hf_k_laplacian: bad arguments");

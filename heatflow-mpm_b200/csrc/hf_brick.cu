@@ -118,13 +118,16 @@ __device__ __forceinline__ void fold(double* v, int lane, int& index) {
 }
 __host__ __device__ constexpr int pow2_above(int k) { return k <= 1 ? 1 : 2 * pow2_above((k + 1) / 2); }
 
-// a / b rounded to double: Newton's iteration for 1 / b from its binary32 value, then the quotient with Markstein's
-// correction (IBM J. Res. Dev. 34(1), 1990; the remainder a - q b is exact with one FMA).  150 cycles from operands to
-// result instead of 410 to 700 for the operator, and the scalars of an iteration wait for two of them.  Operands outside
-// [2^-100, 2^100] take the operator.
+// a / b: Newton's iteration for 1 / b from its binary32 value, then the quotient with Markstein's correction (IBM J. Res.
+// Dev. 34(1), 1990; the remainder a - q b is exact with one FMA).  150 cycles from operands to result instead of 410 to 700
+// for the operator, and the scalars of an iteration wait for two of them.  Markstein's result, that the corrected quotient is
+// rounded correctly, needs a correctly rounded 1 / b, which the iteration does not reach when every bit of b's significand is
+// set (2^k over such a b came out one place low); two steps do not prove it for every other b, so hf_k_quotient compares
+// with the operator.  Those b, and operands outside [2^-100, 2^100], take the operator.
 __device__ __forceinline__ double quotient(double a, double b) {
     const double ab = fabs(b), aa = fabs(a);
-    if (!(ab >= 0x1p-100 && ab <= 0x1p100 && aa >= 0x1p-100 && aa <= 0x1p100)) return a / b;
+    const bool ones = __double2loint(b) == -1 && (__double2hiint(b) & 0xfffff) == 0xfffff;
+    if (!(ab >= 0x1p-100 && ab <= 0x1p100 && aa >= 0x1p-100 && aa <= 0x1p100) || ones) return a / b;
     double y = (double)__frcp_rn((float)b);
     y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
     y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
@@ -1046,6 +1049,11 @@ __global__ void __launch_bounds__(256 * G, 1)
             ws.brick[0] = launch + 1;
         }
     }
+}
+
+// quotient, elementwise (checked against the operator)
+__global__ void k_quotient(int count, const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) out[i] = quotient(a[i], b[i]);
 }
 
 template <bool HEAT>

@@ -80,6 +80,7 @@ __global__ void k_speed_max(const hf_scene* __restrict__ scenes, int s, unsigned
 __global__ void k_laplacian_plain(int n, float h, float alpha, float beta, const float* __restrict__ p,
                                   const float* __restrict__ ax, const float* __restrict__ ay, const float* __restrict__ az,
                                   const float* __restrict__ y, float* __restrict__ out);
+__global__ void k_quotient(int count, const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ out);
 __global__ void k_divide_by(int count, const float* __restrict__ x, float y, float* __restrict__ out);
 __global__ void k_heat_matvec_plain(int n, float h, float dt, float alpha, float beta, const float* __restrict__ x,
                                     const float* __restrict__ kap, const uint8_t* __restrict__ fl,

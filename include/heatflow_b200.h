@@ -217,6 +217,9 @@ int hf_k_heat_matvec(int n, double h, double dt, double alpha, double beta, cons
    sample point by h): out[i] = x[i] / y, correctly rounded, by the kernels' constant-divisor method (a precomputed
    reciprocal pair and one correction; see hf_device.cuh).  For checking that method against IEEE division. */
 int hf_k_divide_by(int count, const float *x, float y, float *out, void *stream);
+/* The division of two inner products that gives alpha and beta in the on-chip CG solves: out[i] = a[i] / b[i] by their
+   method (Newton's reciprocal and one correction; see hf_brick.cu).  For checking that method against IEEE division. */
+int hf_k_quotient(int count, const double *a, const double *b, double *out, void *stream);
 
 /* Failure detection (no counterpart in the reference, whose solves cannot time out).  Every spin-wait of the persistent
    CG kernels -- grid and lane barriers, TMA copies -- gives up after limit_ns (default 2 s), sets

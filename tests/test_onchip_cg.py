@@ -106,3 +106,36 @@ def test_step_numbers_wrap():
         plan.substep(2e-3)
     assert a.read_state().pressure_iters == 1200
     _equal(a, b)
+
+
+def test_quotient_is_the_operators():
+    """The division that gives alpha and beta against numpy's, bit for bit: significands at random, divisors with every bit
+    set and their neighbours, quotients beside the midpoint of two doubles, and any bit patterns at all (zeros, subnormals,
+    infinities and NaNs among them)."""
+    import torch
+    from heatflow_mpm import _lib
+    L = _lib.load()
+    rng = np.random.default_rng(8)
+    N = 1 << 20
+    man = lambda: 1.0 + rng.integers(0, 1 << 52, N) * 2.0 ** -52
+    exp = lambda: np.ldexp(rng.choice([-1.0, 1.0], N), rng.integers(-99, 100, N))
+    ulps = lambda k: rng.integers(0, k, N) * 2.0 ** -52
+    pairs = [(man() * exp(), man() * exp()), ((1.0 + ulps(64)) * exp(), (2.0 - 2.0 ** -52 - ulps(64)) * exp()),
+             ((2.0 - 2.0 ** -52 - ulps(1024)) * exp(), (1.0 + ulps(1024)) * exp())]
+    b = man()
+    mid = man().astype(np.longdouble) + np.longdouble(2.0) ** -53
+    pairs.append(((mid * b.astype(np.longdouble)).astype(np.float64), b))
+    anything = rng.integers(-2 ** 63, 2 ** 63 - 1, (2, N), dtype=np.int64).view(np.float64)
+    pairs.append((anything[0], anything[1]))
+    special = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, 2.0 ** -100, 2.0 ** 100, np.nextafter(2.0 ** 100, 4e30), 1.0, -3.0])
+    pairs.append(tuple(x.ravel() for x in np.meshgrid(special, special)))
+    for a, b in pairs:
+        dev = [torch.as_tensor(np.ascontiguousarray(v), device="cuda") for v in (a, b)]
+        out = torch.empty_like(dev[0])
+        _lib.check(L.hf_k_quotient(out.numel(), dev[0].data_ptr(), dev[1].data_ptr(), out.data_ptr(),
+                                   torch.cuda.current_stream().cuda_stream), "hf_k_quotient")
+        with np.errstate(all="ignore"):
+            want = a / b
+        got = out.cpu().numpy()
+        bad = (got.view(np.int64) != want.view(np.int64)) & ~(np.isnan(got) & np.isnan(want))
+        assert not bad.any(), (int(bad.sum()), a[bad][0].hex(), b[bad][0].hex(), got[bad][0].hex(), want[bad][0].hex())
