@@ -111,6 +111,9 @@ Layout layout(int S, int C, int T) {
     L.mean_part = o;
     o = align_up(o + sizeof(double) * (size_t)C, 256);
     L.streaming = o;
+    // A plan of more tiles than its scenes can have on the chip streams: nothing below is used, nor sized for the rest of them
+    // (not left out, so that a plan whose large scenes are inactive at upload still fits).
+    T = (int)std::min<long long>(T, (long long)S * hf::kUnits * hf::kBrickWideTiles);
     L.brick = o;                     // the on-chip solve: launch, leave and error words
     o = align_up(o + 256, 256);
     L.arrive = o;

@@ -46,6 +46,18 @@ def test_pure_functions_without_gpu():
     assert L.hf_workspace_bytes(1, 864, 864) > 6 * 8 * 864
 
 
+def test_workspace_of_a_scene_too_large_for_the_chip():
+    """The on-chip solves' tables are sized for the tiles that fit there: 148 blocks of 36 for each scene.  A 512^3 scene
+    needs 96 bytes a chunk and tile for the rest, and a plan never needs less room for more tiles."""
+    from heatflow_mpm import _lib
+    L = _lib.load()
+    chunks, tiles, on_chip = L.hf_chunks_for(512), L.hf_tiles_for(512), 148 * 36
+    assert tiles > 10 * on_chip
+    assert L.hf_workspace_bytes(1, chunks, tiles) < 96 * tiles + 7000 * on_chip + (1 << 21)
+    sizes = [L.hf_workspace_bytes(2, chunks, t) for t in (1, 64, 864, on_chip, 2 * on_chip, 2 * on_chip + 1, tiles)]
+    assert sizes == sorted(sizes)
+
+
 def test_record_layout_matches_header(tmp_path):
     if shutil.which("gcc") is None:
         pytest.skip("gcc unavailable")
