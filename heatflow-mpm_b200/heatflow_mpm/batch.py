@@ -98,10 +98,15 @@ class AirScenario:
         return (self.t_amb + rng.uniform(-self.noise, self.noise, (self.n,) * 3)).astype(np.float32)
 
     def device_bytes(self) -> int:
-        """HBM a resident scene of this size takes (fields, statics, CG vectors), for admission control."""
+        """HBM a resident scene of this size takes, for admission control: fields, statics, CG vectors, and its share of two
+        plans' workspaces (the one in use and the one that replaces it when a scene joins or leaves)."""
         n = self.n
         N, NF = n ** 3, (n + 1) * n * n
-        return int(4 * (20 * N + 16 * NF) + N)
+        L = _lib.load()
+        tiles = L.hf_tiles_for(n)
+        # beside smaller scenes every tile of a large one may count (a plan is sized for 148 x 36 tiles a scene at most)
+        share = L.hf_workspace_bytes(1 + tiles // (148 * 36), L.hf_chunks_for(n), tiles)
+        return int(4 * (20 * N + 16 * NF) + N + 2 * share)
 
 
 @functools.lru_cache(maxsize=64)

@@ -121,6 +121,18 @@ def test_admission_respects_slots_and_hbm_budget(monkeypatch):
     assert upload_bytes(small, "host") > upload_bytes(small, "device") == 4 * 32 ** 3
 
 
+def test_device_bytes_count_the_plans():
+    """What the server admits a scene by holds its share of two plans' workspaces beside its fields (20 cell and 16 face
+    arrays of floats, one of bytes), for a plan of any sizes."""
+    from heatflow_mpm import _lib
+    from heatflow_mpm.batch import AirScenario
+    L = _lib.load()
+    for edges in ((12,), (48, 64, 96, 128), (96, 33, 160) * 4, (200, 32)):
+        fields = sum(4 * (20 * n ** 3 + 16 * (n + 1) * n * n) + n ** 3 for n in edges)
+        plan = L.hf_workspace_bytes(len(edges), sum(L.hf_chunks_for(n) for n in edges), sum(L.hf_tiles_for(n) for n in edges))
+        assert sum(AirScenario(n=n).device_bytes() for n in edges) >= fields + 2 * plan, edges
+
+
 # ------------------------------------------------------------------------------------------------------ GPU
 @pytest.fixture(scope="module")
 def cuda():
