@@ -204,99 +204,122 @@ bool any_flag(const hf_plan* p, unsigned f) {
     return false;
 }
 
-// How the on-chip pressure solve shares the blocks among a plan's active scenes: the scenes' jobs in the blocks' common
-// order, the blocks in use, the most tiles that a block owns and the most tiles along k of a scene.
+// How the on-chip solves share the blocks among a plan's active scenes: a team of blocks for each (brick_teams, which every
+// launch forms again: a few us for 64 scenes), and the places of the teams in the blocks' common order (brick_jobs, once at
+// the upload).
+struct BrickTeam {
+    int scene, n, T, blocks, most;   // most: tiles that one of the blocks owns
+};
+// teams, blocks of the launch, the most tiles that a block owns and the most tiles along k of a scene
 struct BrickSchedule {
-    std::vector<int4> jobs;   // (scene, first block, blocks, 0)
-    int blocks = 0, tiles = 0, tk = 0;
+    int jobs, blocks, tiles, tk;
 };
 
 // the most tiles of a block when `blocks` blocks share a scene of T tiles in whole units (hf_brick.cu)
 int brick_tiles(int T, int blocks) {
     const int units = hf::unit_count(T);
     int most = 0;
-    for (int b = 0; b < blocks; ++b)
-        most = std::max(most, hf::unit_first(T, units, (int)((long long)units * (b + 1) / blocks)) -
-                                  hf::unit_first(T, units, (int)((long long)units * b / blocks)));
+    for (int b = 0, first = 0; b < blocks; ++b) {
+        const int end = hf::unit_first(T, units, units * (b + 1) / blocks);
+        most = std::max(most, end - first);
+        first = end;
+    }
     return most;
 }
 
 // False when a scene does not fit: with `cap` kBrickMaxTiles, 148 blocks hold 2220 tiles (an edge of 128 has 2048), with
 // kBrickWideTiles 5328 (an edge of 168 has 5292).
 // Scenes that fit side by side share the blocks in proportion to their tiles.  Otherwise each gets as few blocks as hold
-// it -- the more tiles a block has, the less its reductions weigh -- and the largest come first, each on the contiguous
-// blocks that are free the soonest.
-bool brick_schedule(const hf_plan* p, int sms, int cap, BrickSchedule& out) {
+// it: the more tiles a block has, the less its reductions weigh.  team: room for kMaxScenes.
+bool brick_teams(const hf_plan* p, int sms, int cap, BrickTeam* team, BrickSchedule& out) {
     const int blocks = std::min(sms, hf::kUnits);
-    out = BrickSchedule();
-    struct Want {
-        int scene, n, T, least, blocks;
-    };
-    std::vector<Want> want;
-    long long total = 0;
+    out = BrickSchedule{0, blocks, 0, 0};
+    // the fewest blocks that hold a scene of edge n, and their most tiles: found once for each edge (the divisions of a
+    // search take a few us)
+    struct Fit {
+        int blocks, most;
+    } fits[hf::kBrickEdge + 1] = {};
     int least = 0;
     for (int s = 0; s < p->num_scenes; ++s) {
         const hf_scene& sc = p->scenes_host[s];
         if (!(sc.flags & HF_FLAG_ACTIVE)) continue;
+        if (sc.n < 2 || sc.n > hf::kBrickEdge) return false;
         const int T = tiles_of(sc.n);
-        int nb = (T + cap - 1) / cap;
-        while (nb <= std::min(blocks, T) && brick_tiles(T, nb) > cap) ++nb;
-        if (nb > std::min(blocks, T)) return false;
-        want.push_back(Want{s, sc.n, T, nb, nb});
-        total += T;
-        least += nb;
+        Fit& fit = fits[sc.n];
+        if (!fit.blocks) {
+            fit.blocks = (T + cap - 1) / cap;
+            while (fit.blocks <= std::min(blocks, T) && (fit.most = brick_tiles(T, fit.blocks)) > cap) ++fit.blocks;
+            if (fit.blocks > std::min(blocks, T)) return false;
+        }
+        team[out.jobs++] = BrickTeam{s, sc.n, T, fit.blocks, fit.most};
+        least += fit.blocks;
         out.tk = std::max(out.tk, (sc.n + hf::kTK - 1) / hf::kTK);
     }
-    if (want.empty()) return false;
+    if (!out.jobs) return false;
     if (least <= blocks) {
         // side by side: the blocks that are left go, one at a time, to the scene whose blocks own the most tiles
-        for (int left = blocks - least; left > 0; --left) {
-            Want* most = nullptr;
-            for (Want& w : want)
-                if (w.blocks < std::min(blocks, w.T) && (!most || (long long)w.T * most->blocks > (long long)most->T * w.blocks)) most = &w;
+        for (; least < blocks; ++least) {
+            BrickTeam* most = nullptr;
+            for (BrickTeam* w = team; w < team + out.jobs; ++w)
+                if (w->blocks < std::min(blocks, w->T) && (!most || (long long)w->T * most->blocks > (long long)most->T * w->blocks)) most = w;
             if (!most) break;
             ++most->blocks;
         }
+        out.blocks = least;
+        for (int q = 0; q < out.jobs; ++q) team[q].most = brick_tiles(team[q].T, team[q].blocks);
     }
-    std::stable_sort(want.begin(), want.end(), [](const Want& a, const Want& b) { return a.T > b.T; });
-    std::vector<double> until(blocks, 0.0);
-    for (const Want& w : want) {
-        int at = 0;
+    for (int q = 0; q < out.jobs; ++q) out.tiles = std::max(out.tiles, team[q].most);
+    return true;
+}
+
+bool brick_teams(const hf_plan* p, int sms, BrickTeam* team, BrickSchedule& out) {
+    return brick_teams(p, sms, hf::kBrickMaxTiles, team, out) || brick_teams(p, sms, hf::kBrickWideTiles, team, out);
+}
+
+// The jobs (scene, first block, blocks, the most tiles of a block): the largest scenes come first, each on the contiguous
+// blocks that are free the soonest.
+std::vector<int4> brick_jobs(const BrickTeam* team, const BrickSchedule& sched) {
+    std::vector<BrickTeam> order(team, team + sched.jobs);
+    std::stable_sort(order.begin(), order.end(), [](const BrickTeam& a, const BrickTeam& b) { return a.T > b.T; });
+    std::vector<double> until(sched.blocks, 0.0);
+    std::vector<int> high(sched.blocks);   // blocks of the window, each busy for longer than all after it
+    std::vector<int4> jobs;
+    for (const BrickTeam& w : order) {
+        int at = 0, head = 0, tail = 0;
         double best = 0.0;
-        for (int f = 0; f + w.blocks <= blocks; ++f) {
-            const double t = *std::max_element(until.begin() + f, until.begin() + f + w.blocks);
+        for (int e = 0; e < sched.blocks; ++e) {   // the window's last block
+            while (tail > head && until[high[tail - 1]] <= until[e]) --tail;
+            high[tail++] = e;
+            const int f = e - w.blocks + 1;
+            if (f < 0) continue;
+            if (high[head] < f) ++head;
+            const double t = until[high[head]];
             if (f == 0 || t < best) {
                 best = t;
                 at = f;
             }
         }
         // an iteration takes about 1.6 us of exchanges and 0.35 us a tile; iterations grow like the edge
-        const int most = brick_tiles(w.T, w.blocks);
-        std::fill(until.begin() + at, until.begin() + at + w.blocks, best + w.n * (1.6 + 0.35 * most));
-        out.jobs.push_back(make_int4(w.scene, at, w.blocks, 0));
-        out.blocks = std::max(out.blocks, at + w.blocks);
-        out.tiles = std::max(out.tiles, most);
+        std::fill(until.begin() + at, until.begin() + at + w.blocks, best + w.n * (1.6 + 0.35 * w.most));
+        jobs.push_back(make_int4(w.scene, at, w.blocks, w.most));
     }
-    return true;
-}
-
-bool brick_schedule(const hf_plan* p, int sms, BrickSchedule& out) {
-    return brick_schedule(p, sms, hf::kBrickMaxTiles, out) || brick_schedule(p, sms, hf::kBrickWideTiles, out);
+    return jobs;
 }
 
 // The on-chip solve of a plan whose scenes all fit.  HF_OK after launching, -1 when it does not apply.
 int launch_brick(const hf_plan* p, DeviceInfo* d, bool heat, double dt, void* stream) {
     if (!(p->options & HF_PLAN_MAPS_READY) || p->workspace_bytes < layout(p->num_scenes, p->num_chunks, p->num_tiles).total) return -1;
+    static thread_local BrickTeam team[hf::kMaxScenes];
     BrickSchedule sched;
-    if (!brick_schedule(p, d->sms, sched)) return -1;
+    if (!brick_teams(p, d->sms, team, sched)) return -1;
     for (int s = 0; s < p->num_scenes; ++s) {
         const hf_scene& sc = p->scenes_host[s];
         if ((sc.flags & HF_FLAG_ACTIVE) && (!sc.pdiag || !sc.hdiag || !sc.cg_r || !sc.cg_z || !sc.cg_Ap)) return -1;   // scratch of the larger variants
     }
     hf::BrickLaunch bl;
     std::memset(&bl, 0, sizeof bl);
-    bl.jobs = (int)sched.jobs.size();
-    bl.job0 = sched.jobs[0];
+    bl.jobs = sched.jobs;
+    bl.job0 = make_int4(team[0].scene, 0, team[0].blocks, sched.tiles);   // of several jobs the places are in the workspace
     bl.tiles = sched.tiles;
     // A block's run of tiles is contiguous in (k, i, j): at most 2 tk of its i faces, all of its j faces and the two k
     // faces at the run's ends border other blocks.
@@ -501,17 +524,31 @@ int hf_plan_upload(hf_plan* p, void* stream) {
     }
     HF_CUDA(cudaMemcpyAsync(b + L.maps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice, S(stream)),
             "upload TMA descriptors");
-    // the on-chip pressure solve's jobs (launch_brick recomputes the same schedule)
+    // the on-chip solves' jobs (launch_brick forms the same teams)
+    std::vector<BrickTeam> team(p->num_scenes);
+    std::vector<int4> jobs;
     BrickSchedule sched;
     DeviceInfo* d = nullptr;
     int drc = device_info(&d);
     if (drc) return drc;
-    if (p->num_tiles && brick_schedule(p, d->sms, sched))
-        HF_CUDA(cudaMemcpyAsync(b + L.jobs, sched.jobs.data(), sizeof(int4) * sched.jobs.size(), cudaMemcpyHostToDevice, S(stream)),
-                "upload jobs");
+    if (p->num_tiles && brick_teams(p, d->sms, team.data(), sched)) {
+        jobs = brick_jobs(team.data(), sched);
+        HF_CUDA(cudaMemcpyAsync(b + L.jobs, jobs.data(), sizeof(int4) * jobs.size(), cudaMemcpyHostToDevice, S(stream)), "upload jobs");
+    }
     HF_CUDA(cudaStreamSynchronize(S(stream)), "cudaStreamSynchronize(plan upload)");
     p->options |= HF_PLAN_MAPS_READY;
     return HF_OK;
+}
+
+int hf_plan_jobs(const hf_plan* p, int sms, int* jobs) {
+    if (!p || !p->scenes_host || p->num_scenes <= 0 || p->num_scenes > hf::kMaxScenes || sms < 1)
+        return -fail(HF_ERR_ARG, "hf_plan_jobs: bad arguments");
+    if ((p->options & HF_PLAN_STREAMING_CG) || any_flag(p, HF_FLAG_DEFECT_CORRECTION)) return 0;
+    std::vector<BrickTeam> team(p->num_scenes);
+    BrickSchedule sched;
+    if (!brick_teams(p, sms, team.data(), sched)) return 0;
+    if (jobs) std::memcpy(jobs, brick_jobs(team.data(), sched).data(), sizeof(int4) * sched.jobs);
+    return sched.jobs;
 }
 
 int hf_obstacle_fields(const hf_plan* p, int all_scenes, void* stream) {

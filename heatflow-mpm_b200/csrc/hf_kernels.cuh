@@ -44,6 +44,7 @@ struct Workspace {
 
 constexpr int kBrickMaxTiles = 15;   // tiles of an on-chip solve's block with r, A p and x on the chip at most,
 constexpr int kBrickWideTiles = 36;  // with p alone
+constexpr int kBrickEdge = 168;      // the largest edge whose tiles 148 such blocks hold
 constexpr int kHaloEntries = 832;    // cells on the six faces of a tile, face by face
 
 // Launch of the on-chip pressure solve: `tiles` is the most that a block owns; halo pages of 1024 floats (for i faces, for

@@ -110,6 +110,7 @@ def load():
     L.hf_k_laplacian.argtypes = [C.c_int, C.c_double, C.c_double, C.c_double] + [_P] * 6 + [_P]
     L.hf_k_heat_matvec.argtypes = [C.c_int, C.c_double, C.c_double, C.c_double, C.c_double] + [_P] * 5 + [_P]
     L.hf_k_divide_by.argtypes = [C.c_int, _P, C.c_float, _P, _P]
+    L.hf_plan_jobs.argtypes = [C.POINTER(Plan), C.c_int, _P]
     L.hf_k_quotient.argtypes = [C.c_int, _P, _P, _P, _P]
     L.hf_set_wait_limit.argtypes = [C.c_ulonglong, C.c_int]
     if L.hf_abi_version() != 1:

@@ -346,6 +346,16 @@ class ScenePlan:
             self.host[i] = sc.record
         _lib.check(self.L.hf_plan_upload(C.byref(self.plan), self.stream()), "hf_plan_upload")
 
+    def onchip_jobs(self):
+        """How the on-chip CG solves serve the plan: (scene, first block, blocks, most tiles of a block) in the order in which
+        a block takes its scenes; empty when the plan's solves stream."""
+        sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+        jobs = (C.c_int32 * (4 * len(self.scenes)))()
+        count = self.L.hf_plan_jobs(C.byref(self.plan), sms, jobs)
+        if count < 0:
+            _lib.check(-count, "hf_plan_jobs")
+        return [tuple(jobs[4 * q:4 * q + 4]) for q in range(count)]
+
     def _call(self, name, *args):
         if any(sc.dirty for sc in self.scenes):
             self.upload()

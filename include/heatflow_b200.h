@@ -163,6 +163,11 @@ int hf_tiles_for(int n);
  * device, fills plan.num_chunks/num_tiles and sets HF_PLAN_MAPS_READY.  Blocking: the stream is synchronised before
  * return (set-up call, not for the per-substep path).  Call it again whenever a scene's buffers change. */
 int hf_plan_upload(hf_plan *plan, void *stream);
+/* How the on-chip CG solves would serve the plan's active scenes on a device of `sms` SMs: the number of jobs (scenes), 0 when
+ * the plan streams (a scene that does not fit, the defect correction, HF_PLAN_STREAMING_CG), negative on bad arguments.
+ * jobs (room for num_scenes quadruples, or NULL): scene, first block, blocks and the most tiles that one of them owns, in the
+ * order in which a block takes its scenes.  Host arithmetic only. */
+int hf_plan_jobs(const hf_plan *plan, int sms, int32_t *jobs);
 
 /* --------------------------------------------------------------------------------- per-substep stages (batched) */
 /* solver.py:65-72 + grid.py:202-213 + grid.py:46-67 + heat.py:44-47: obstacle fields of every scene -- particle
