@@ -3,11 +3,12 @@
 ``AirScenario`` describes one air-only scene (grid edge, heater, fan, optional static solid sphere).  ``AirBatch``
 builds the device scenes, one plan over all of them (scene table + chunk and tile tables: the kernels walk the tables,
 so scenes of different n share every launch), optionally captures K substeps in one CUDA graph, and reports per-scene
-state.  The CG solves of a batch run in the streaming persistent kernels with per-scene convergence masking: a scene
-that has converged stops iterating while the others continue.  Results are bit-identical to each scene run alone.
+state.  The CG solves of a batch run on the chip, a team of blocks for each scene, when every scene fits there (edges up to
+168), and otherwise in the streaming persistent kernels; a scene that has converged stops iterating while the others
+continue.  Results are bit-identical to each scene run alone.
 
-``autotune`` picks the launch shape of the CG solves for a batch -- blocks of the streaming kernel, the cells of one
-scene group (a group's CG vectors should stay in L2) and the lanes that solve groups side by side -- by timing
+``autotune`` picks the launch shape of the streaming solves for a batch that needs them -- blocks of the kernel, the cells
+of one scene group (a group's CG vectors should stay in L2) and the lanes that solve groups side by side -- by timing
 candidates on the device; every candidate computes the same bits, so tuning never changes results.  Choices are cached
 per GPU and batch signature in a JSON file.
 """
@@ -215,10 +216,14 @@ def _signature(scenes):
 
 
 def autotune(batch: AirBatch, dt=2e-3, reps=3, candidates=None, cache=True):
-    """Time launch-shape candidates (persistent_blocks, group_cells, lanes) of the CG solves on this batch and keep
-    the fastest.  Every candidate times the same `reps` substeps from the batch's current state (restored before each
+    """Time launch-shape candidates (persistent_blocks, group_cells, lanes) of the streaming CG solves on this batch and
+    keep the fastest.  Every candidate times the same `reps` substeps from the batch's current state (restored before each
     one, after a warm-up substep), and the batch is left as it was found.  Returns (the chosen triple,
-    {"blocks/cells/lanes": ms per substep})."""
+    {"blocks/cells/lanes": ms per substep}).  The on-chip solves have no such choice: a batch that they serve returns at
+    once with the triple that it has and no timings (candidates that the caller names are timed all the same)."""
+    if not candidates and batch.plan.onchip_jobs():
+        plan = batch.plan
+        return (plan.plan.persistent_blocks, plan.plan.group_cells, plan.lanes), {}
     sms = torch.cuda.get_device_properties(batch.device).multi_processor_count
     name = torch.cuda.get_device_name(batch.device)
     key = f"{name}|{_signature(batch.scenes)}"

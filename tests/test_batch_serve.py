@@ -254,6 +254,21 @@ def test_autotune_keeps_results(cuda):
 
 
 @pytest.mark.gpu
+def test_autotune_of_a_batch_on_the_chip_runs_nothing(cuda):
+    """The on-chip solves have no launch shape to tune: no substep runs and the plan keeps its shape.  A batch with a scene
+    that streams is still tuned."""
+    from heatflow_mpm.batch import AirBatch, AirScenario, autotune
+    b = AirBatch([AirScenario(n=24, power=200.0), AirScenario(n=33)], lanes=2)
+    ran = []
+    b.plan.substep = ran.append
+    assert autotune(b, cache=False) == ((0, 0, 2), {}) and not ran
+    big = AirBatch([AirScenario(n=24), AirScenario(n=169)])
+    big.plan.substep = ran.append
+    best, timings = autotune(big, reps=1, cache=False)
+    assert len(timings) == 30 and len(ran) == 60 and "/".join(map(str, best)) in timings
+
+
+@pytest.mark.gpu
 def test_served_failure_is_reported_for_that_request_only(cuda):
     """Three requests served together; after the first batched substep a NaN is written on the host into the middle
     request's temperature.  The server's status check finds HF_SCENE_NONFINITE, that request leaves the batch as
