@@ -68,19 +68,19 @@ def parse():
     ap.add_argument("--ref-seconds", type=float, default=60.0, help="budget of the timed CPU reference arm")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-extras", action="store_true", help="plain line without the batched/served summaries")
-    ap.add_argument("--resident-tiles", type=int, default=0, help="plain: tiles per group of the resident CG (0: auto)")
+    ap.add_argument("--resident-tiles", type=int, default=0, help="plain: accepted, without effect (the on-chip CG chooses)")
     ap.add_argument("--no-graph", action="store_true", help="plain: time eager launches instead of one graph replay")
     ap.add_argument("--streaming", default="none", choices=["none", "heat", "both"],
-                    help="plain: CG solves in the streaming kernel instead of the resident one")
+                    help="plain: CG solves in the streaming kernel instead of the on-chip one")
     ap.add_argument("--persistent-blocks", type=int, default=0, help="plain: grid of the streaming CG kernel")
-    ap.add_argument("--no-tma", action="store_true", help="plain: resident pressure CG without the TMA-staged stencil")
+    ap.add_argument("--no-tma", action="store_true", help="plain, --streaming both: pressure CG without TMA staging")
     ap.add_argument("--cg", default="single-reduction", choices=["classic", "single-reduction"],
                     help="plain: the pressure solve that HeatflowMPM is asked for (both are served by the on-chip classic "
                          "Jacobi-PCG)")
     ap.add_argument("--scenes", type=int, default=64, help="batched: scenes in the ensemble")
     ap.add_argument("--graph-steps", type=int, default=10, help="batched: substeps per captured CUDA graph")
     ap.add_argument("--edges", default="32,48,64,96,128", help="batched: grid edges the ensemble draws from")
-    ap.add_argument("--no-autotune", action="store_true", help="batched: default launch shape, no tuning")
+    ap.add_argument("--no-autotune", action="store_true", help="batched: default launch shape of the streaming CG, no tuning")
     ap.add_argument("--launch", default=None, help="batched: fixed CG launch shape 'blocks,group_cells,lanes'")
     ap.add_argument("--serve-seconds", type=float, default=60.0, help="served: length of the trace window")
     ap.add_argument("--rate", type=float, default=20.0, help="served: mean arrivals per second")
@@ -349,6 +349,30 @@ def roofline(achieved_gbs, peaks, **extra):
     return out
 
 
+def pressure_kernel(plan, mean_iters=None):
+    """Which kernel solves the plan's pressure, what bounds it and, where it was measured (DRAM bytes of a single 96^3 scene's
+    launch), its traffic; the path is the library's own choice (hf_plan_jobs)."""
+    jobs = plan.onchip_jobs()
+    if not jobs:
+        tma = all(sc.n % 4 == 0 for sc in plan.scenes) and not plan.plan.options & 2   # HF_PLAN_NO_TMA
+        return {"kernel": f"k_pcg<false, {str(tma).lower()}> (streaming persistent pressure Jacobi-PCG + projection over the scene "
+                          f"table{', TMA-staged double-buffered tile boxes' if tma else ''})",
+                "bound": "hbm", "traffic": None}
+    most = max(j[3] for j in jobs)
+    chip = "CG state on the chip" if most <= 15 else "p on the chip, r, A p and x through L2"
+    out = {"kernel": f"k_brick (pressure Jacobi-PCG + projection, one cooperative launch, a team of blocks per scene, up to {most} "
+                     f"tiles a block, {chip}, tagged exchanges)",
+           "bound": "latency and issue (achieved: bytes of the streaming formulation, most of which stay on the chip)",
+           "traffic": None}
+    if mean_iters is not None and [sc.n for sc in plan.scenes] == [96]:
+        try:
+            prof = json.load(open(os.path.join(ROOT, "profiles", "pressure_cg_chip_96.json")))
+            out["traffic"] = prof["dram_bytes_per_iteration"] * mean_iters + prof.get("dram_bytes_fixed", 0.0)
+        except (OSError, ValueError, KeyError):
+            pass
+    return out
+
+
 def stage_breakdown(plan, stages, substeps=20):
     """Mean device time of every stage of a substep, from CUDA events around each stage launch over `substeps`
     substeps run after the timed region (the stages in substep order, warm caches as in the timed run)."""
@@ -495,15 +519,7 @@ def bench_plain(args, dev, rank, world, local):
     # ---- roofline of the dominant kernel (pressure CG + projection) and of the whole substep
     peaks = load_peaks()
     cg_bytes = pressure_bytes_per_launch(N, p_iters / steps)
-    traffic = None
-    try:
-        prof = json.load(open(os.path.join(ROOT, "profiles", "pressure_cg_chip_96.json")))
-        traffic = prof["dram_bytes_per_iteration"] * (p_iters / steps) + prof.get("dram_bytes_fixed", 0.0)
-    except (OSError, ValueError, KeyError):
-        pass
-    kernel = ("k_brick<3, 2, false> (pressure Jacobi-PCG + projection, one persistent cooperative launch, CG state in registers "
-              "and shared memory, tagged exchanges)")
-    roof = roofline(cg_bytes / (cg_ms / steps / 1000.0) / 1e9, peaks, traffic=traffic, kernel=kernel,
+    roof = roofline(cg_bytes / (cg_ms / steps / 1000.0) / 1e9, peaks, **pressure_kernel(plan, p_iters / steps),
                     bytes_per_launch=cg_bytes, ms_per_launch=cg_ms / steps, mean_pressure_iters=p_iters / steps)
     sb = substep_bytes(N, h_iters / steps, p_iters / steps, True)
     sub_gbs = sb / (el_ms / steps / 1000.0) / 1e9
@@ -543,7 +559,7 @@ def bench_plain(args, dev, rank, world, local):
                         "cell_updates_per_s": value * N, "substep_status": int(st1.status),
                         "substep_roofline": sub_roof, "stage_ms": stage_ms,
                         "timed_launches": "one CUDA-graph replay of the K substeps" if use_graph else "eager launches",
-                        "pressure_cg": args.cg},
+                        "pressure_cg": "classic", "cg_option": args.cg},
             "parity": parity,
             "roofline": roof, "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": launches_per_step * steps, "clocks": ck}
 
@@ -685,8 +701,7 @@ def bench_batched(args, dev, rank, world, local, steps, warmup, cpu_sample=True)
     cg_bytes = sum(pressure_bytes_per_launch(s.n ** 3, (b.total_pressure_iters - a.total_pressure_iters) / B)
                    for s, a, b in zip(mine, sa, sbk))
     peaks = load_peaks()
-    roof = roofline(cg_bytes / (cg_ms / 1000.0) / 1e9, peaks, traffic=None,
-                    kernel="k_brick<3, 5, false> (pressure Jacobi-PCG + projection, one team of blocks per scene, CG state on the chip)",
+    roof = roofline(cg_bytes / (cg_ms / 1000.0) / 1e9, peaks, **pressure_kernel(plan),
                     bytes_per_launch=cg_bytes, ms_per_launch=cg_ms, measured_on="rank 0 stage breakdown, 10 substeps")
     sub_gbs = sb / (el_ms / steps / 1000.0) / 1e9
     # ---- end to end through the public API: AirBatch.substep per substep, every scene's status block read back
@@ -729,7 +744,7 @@ def bench_batched(args, dev, rank, world, local, steps, warmup, cpu_sample=True)
                                    f"h=0.48 m/edge, box heater x U(0.05,0.2) m, 100-800 W, fan 0-3 m/s, dt=2 ms, "
                                    f"pressure tol 1e-4, heat tol 1e-6",
                        "scenes": args.scenes, "cells": int(cells), "graph_substeps": G, "persistent_blocks": pb,
-                       "group_cells": gc, "lanes": lanes,
+                       "group_cells": gc, "lanes": lanes, "cg": "on-chip" if batch.plan.onchip_jobs() else "streaming",
                        "autotune_ms": tune, "parallelism": f"scene-sharded x{world}",
                        "l2": f"{cells * 4 * 40 / 1e9:.1f} GB of scene state > 126 MB L2 (inputs larger than L2)",
                        "scene_substeps_per_s": len(scs_all) * steps / (el_ms / 1000.0),

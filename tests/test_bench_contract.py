@@ -176,3 +176,18 @@ def test_clock_sampler_with_a_fake_nvml(monkeypatch):
     cs = bench.ClockSampler(0)
     cs.start()
     assert cs.stop() is None
+
+
+def test_bench_names_the_pressure_kernel_that_runs():
+    """The roofline's kernel, bound and traffic follow the path that the plan takes: DRAM traffic was measured for the on-chip
+    solve of one 96^3 scene only, and a plan that streams names the streaming kernel."""
+    from types import SimpleNamespace as NS
+    import bench
+    plan = lambda edges, jobs, options=0: NS(scenes=[NS(n=n) for n in edges], plan=NS(options=options), onchip_jobs=lambda: jobs)
+    one = bench.pressure_kernel(plan((96,), [(0, 0, 148, 6)]), 45.0)
+    assert "k_brick" in one["kernel"] and "6 tiles" in one["kernel"] and "latency" in one["bound"] and one["traffic"] > 0
+    wide = bench.pressure_kernel(plan((160, 32), [(0, 0, 140, 28), (1, 140, 8, 4)]))
+    assert "k_brick" in wide["kernel"] and "28 tiles" in wide["kernel"] and "through L2" in wide["kernel"] and wide["traffic"] is None
+    for edges, options, tma in (((96,), 0, True), ((96, 33), 0, False), ((96,), 2, False)):
+        got = bench.pressure_kernel(plan(edges, [], options), 45.0)
+        assert got["kernel"].startswith(f"k_pcg<false, {str(tma).lower()}>") and got["bound"] == "hbm" and got["traffic"] is None
