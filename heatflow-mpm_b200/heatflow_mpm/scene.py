@@ -252,9 +252,9 @@ def recording(graph, stream):
     copies meanwhile).  torch.cuda.graph would also collect garbage and give all cached memory back to the driver -- from
     tens of milliseconds to over a second -- which a recording that allocates nothing does not need; it must only not be
     interrupted by a collection that frees CUDA objects.  A graph that this one replaces is no longer in flight: the
-    device is synchronised first."""
-    torch.cuda.synchronize(stream.device)
+    device is synchronised first, and not while another thread records, whose recording that would end."""
     with _recording:
+        torch.cuda.synchronize(stream.device)
         collecting = gc.isenabled()
         gc.disable()
         try:
