@@ -32,6 +32,7 @@ namespace hf {
 // k_pcg's `red` holds kRedComps x 32 doubles: up to 9 components of one sum, or the 8 warps' sums of the group_sums of 36
 // scenes and one component.
 constexpr int kRedComps = 9;
+constexpr int kPlaces = 64;          // tiles of a block whose partials' places a solve keeps (those of more are found each time)
 constexpr int kMaxCorrections = 2;   // restarts of one solve by the outer defect correction
 
 // Barrier of nblocks blocks (the grid, or one lane of it) with a bounded wait.  Thread 0 publishes the block's writes with a release reduction (cumulative over
@@ -63,16 +64,46 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned& epoch, int
 // obtains the same bits.  Tile partials (cs: the plan's tile count): thread u adds the tiles of unit u (unit_first) when
 // the scene is one that the on-chip solve takes; of a larger scene (whose runs of 16 tiles and more would be as many
 // dependent round trips), and of the per-chunk rhs sums (cs = 0, one component), thread t adds items t, t + 256, ...
+//
+// A unit's partials are stored where its thread's loads are coalesced with its neighbours' (part_at): partial q of unit u at
+// q * units + u, the last ones of the longer units behind these.  Read from the unit's own run of tiles, every sector was
+// fetched up to four times.  us per iteration with the defect correction (whole substep), strided sums / runs / now: 75^3
+// 20.2 / 21.4 / 20.8, 96^3 20.1 / 20.7 / 20.1, 128^3 36.4 / 39.8 / 37.6, 160^3 71.8 / 81.5 / 74.4, 168^3 96.1 / 105.1 / 96.0;
+// ms per substep of 40 scenes of 48^3 18.9 / 20.1 / 18.4.
 struct Run {
-    int first, end, step;
+    int first, step, count, last;   // items first, first + step, ...; the last one (count - 1) at `last`
+    __device__ __forceinline__ int at(int q) const { return q < count - 1 ? first + q * step : last; }
 };
+
+// (Of up to kUnits tiles every unit is one: the strided sum is the same.)
+__device__ __forceinline__ bool in_units(int T) { return T > kUnits && T <= kUnits * kBrickWideTiles; }
+
+// first tile of unit u of such a scene: unit_first(T, kUnits, u) with a constant divisor (a division by a variable costs 150
+// cycles, four times an iteration)
+__device__ __forceinline__ int unit_start(int T, int u) { return T * u / kUnits; }
 
 // the items of [b, e) that this thread adds
 __device__ __forceinline__ Run thread_run(int b, int e, int cs) {
-    const int t = threadIdx.x, T = e - b, units = unit_count(T);
-    if (cs == 0 || T > kUnits * kBrickWideTiles) return Run{b + t, t < kThreads ? e : b, kThreads};
-    if (t >= units) return Run{b, b, 1};
-    return Run{b + unit_first(T, units, t), b + unit_first(T, units, t + 1), 1};
+    const int t = threadIdx.x, T = e - b;
+    if (cs == 0 || !in_units(T)) {
+        const int count = t < kThreads && t < T ? (T - t + kThreads - 1) / kThreads : 0;
+        return Run{b + t, kThreads, count, b + t + (count - 1) * kThreads};
+    }
+    if (t >= kUnits) return Run{b, 0, 0, b};
+    const int least = T / kUnits, first = unit_start(T, t), count = unit_start(T, t + 1) - first;
+    return Run{b + t, kUnits, count, b + (count > least ? least * kUnits + first - t * least : t + (least - 1) * kUnits)};
+}
+
+// Where the partials of tile c of a scene are kept.  Some 300 cycles for one thread, so a solve finds its tiles' places once
+// (kPlaces; in global memory their loads took 6 us an iteration at 180^3).
+__device__ __forceinline__ int part_at(const int* __restrict__ tile_begin, int scene, int c) {
+    const int b = tile_begin[scene], T = tile_begin[scene + 1] - b, i = c - b;
+    if (!in_units(T)) return c;
+    int u = (int)(__fdividef((float)(i * kUnits), (float)T));   // within one of the unit that holds i
+    u -= unit_start(T, u) > i;
+    u += unit_start(T, u + 1) <= i;
+    const int first = unit_start(T, u), q = i - first, least = T / kUnits;
+    return b + (q < least ? q * kUnits + u : least * kUnits + first - u * least);
 }
 
 template <int K, int U = 4>
@@ -82,15 +113,15 @@ __device__ __forceinline__ void scene_sums(const double* __restrict__ buf, int b
 #pragma unroll
     for (int q = 0; q < K; ++q) tot[q] = 0.0;
     const Run run = thread_run(b, e, cs);
-    if (run.first < run.end) {
+    {
         // U items at a time are loaded (an absent one as +0.0, which leaves a sum that started at +0.0 unchanged) before
         // they are added, so their L2 round trips overlap instead of each waiting for the previous addition
-        for (int c = run.first; c < run.end; c += U * run.step) {
+        for (int c = 0; c < run.count; c += U) {
             double v[U][K];
 #pragma unroll
             for (int u = 0; u < U; ++u)
 #pragma unroll
-                for (int q = 0; q < K; ++q) v[u][q] = c + u * run.step < run.end ? buf[comp[q] * cs + c + u * run.step] : 0.0;
+                for (int q = 0; q < K; ++q) v[u][q] = c + u < run.count ? buf[comp[q] * cs + run.at(c + u)] : 0.0;
 #pragma unroll
             for (int u = 0; u < U; ++u)
 #pragma unroll
@@ -136,17 +167,24 @@ __device__ __forceinline__ void group_sums(const double* __restrict__ buf, const
             double acc[K];
 #pragma unroll
             for (int k = 0; k < K; ++k) acc[k] = 0.0;
-            const Run run = thread_run(b, e, cs);
-            for (int c = run.first; c < run.end; c += 4 * run.step) {
-                double v[4][K];
+            if (e - b <= kUnits) {   // one item a thread: small scenes in numbers spend their time here
+                if (b + lt < e)
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
+                    for (int k = 0; k < K; ++k) acc[k] = buf[comp[k] * cs + b + lt];
+            } else {
+                const Run run = thread_run(b, e, cs);
+                constexpr int U = K == 1 ? 14 : 8;   // in flight: as many as fit the registers (14 pairs spill, 39.0 us at 128^3)
+                for (int c = 0; c < run.count; c += U) {
+                    double v[U][K];
 #pragma unroll
-                    for (int k = 0; k < K; ++k) v[u][k] = c + u * run.step < run.end ? buf[comp[k] * cs + c + u * run.step] : 0.0;
+                    for (int u = 0; u < U; ++u)
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
+                        for (int k = 0; k < K; ++k) v[u][k] = c + u < run.count ? buf[comp[k] * cs + run.at(c + u)] : 0.0;
 #pragma unroll
-                    for (int k = 0; k < K; ++k) acc[k] += v[u][k];
+                    for (int u = 0; u < U; ++u)
+#pragma unroll
+                        for (int k = 0; k < K; ++k) acc[k] += v[u][k];
+                }
             }
 #pragma unroll
             for (int k = 0; k < K; ++k) {
@@ -435,14 +473,15 @@ template <class Issue, class Work>
 __device__ __forceinline__ void pipelined_tiles(int first, int end, int step, const LocalScene* loc, int scene_lo,
                                                 const TileItem* __restrict__ tiles, float* slots,
                                                 unsigned long long* mbar, unsigned& ph, int* err, Issue issue, Work work) {
-    auto next_live = [&](int c) {
-        while (c < end && !loc[tiles[c].scene - scene_lo].live) c += step;
+    auto next_live = [&](int c, int& nth) {
+        while (c < end && !loc[tiles[c].scene - scene_lo].live) c += step, ++nth;
         return c;
     };
-    int cur = next_live(first), si = 0;
+    int nth = 0, si = 0, cur = next_live(first, nth);
     if (cur < end && threadIdx.x == 0) issue(cur, slots, &mbar[0]);
     while (cur < end) {
-        const int nxt = next_live(cur + step);
+        int nth_nxt = nth + 1;
+        const int nxt = next_live(cur + step, nth_nxt);
         if (nxt < end && threadIdx.x == 0) issue(nxt, slots + (si ^ 1) * kSlotFloats, &mbar[si ^ 1]);
         const unsigned phase = (ph >> si) & 1u;
         if (!mbar_wait(&mbar[si], phase)) {
@@ -450,8 +489,9 @@ __device__ __forceinline__ void pipelined_tiles(int first, int end, int step, co
             mbar_wait(&mbar[si], phase);
         }
         ph ^= 1u << si;
-        work(cur, slots + si * kSlotFloats);
+        work(cur, slots + si * kSlotFloats, nth);
         cur = nxt;
+        nth = nth_nxt;
         si ^= 1;
     }
 }
@@ -468,11 +508,13 @@ template <bool HEAT, bool TMA>
 __device__ bool solve_group(const hf_scene* __restrict__ scenes, const TileItem* __restrict__ tiles, const int4 grp,
                             int lb, int nlb, unsigned* bar, unsigned& epoch, double dt_d, const Workspace& ws,
                             double* red, LocalScene* loc, unsigned char* s_par, int* s_any, float* slots,
-                            unsigned long long* mbar, unsigned& ph) {
+                            unsigned long long* mbar, unsigned& ph, int* place) {
     const int scene_lo = grp.x, scene_hi = grp.y, tile_lo = grp.z, tile_hi = grp.w;
     const int ns = scene_hi - scene_lo;
     double* bufA = ws.partA;
     double* bufB = ws.partB;
+    // part_at of this block's nth tile (thread 0)
+    auto placed = [&](int nth, int scene, int c) { return nth < kPlaces ? place[nth] : part_at(ws.tile_begin, scene, c); };
     const float dt = (float)dt_d;
     const int lt = threadIdx.x;
     const int first = tile_lo + lb;
@@ -494,7 +536,7 @@ __device__ bool solve_group(const hf_scene* __restrict__ scenes, const TileItem*
         }
     }
     __syncthreads();
-    for (int c = first; c < tile_hi; c += nlb) {
+    for (int c = first, nth = 0; c < tile_hi; c += nlb, ++nth) {
         const TileItem ti = tiles[c];
         const hf_scene& S = scenes[ti.scene];
         const int n = S.n, par = s_par[ti.scene - scene_lo];
@@ -518,9 +560,11 @@ __device__ bool solve_group(const hf_scene* __restrict__ scenes, const TileItem*
         }
         group_sum<3>(part, red);
         if (lt == 0) {
-            bufB[c] = part[0];
-            bufB[1 * ws.tiles + c] = part[1];
-            bufB[2 * ws.tiles + c] = part[2];
+            const int at = part_at(ws.tile_begin, ti.scene, c);
+            if (nth < kPlaces) place[nth] = at;
+            bufB[at] = part[0];
+            bufB[1 * ws.tiles + at] = part[1];
+            bufB[2 * ws.tiles + at] = part[2];
         }
     }
     if (!(ok = grid_barrier(bar, epoch, ws.err, nlb))) goto done;
@@ -570,7 +614,7 @@ __device__ bool solve_group(const hf_scene* __restrict__ scenes, const TileItem*
                     tma_load_3d(slot + 2 * kBZ + kBX + kBY, &M[5], ti.k0, ti.j0, ti.i0, mb);
                 }
             };
-            auto work = [&](int c, float* slot) {
+            auto work = [&](int c, float* slot, int nth) {
                 const TileItem ti = tiles[c];
                 const LocalScene& L = loc[ti.scene - scene_lo];
                 const hf_scene& S = scenes[ti.scene];
@@ -607,11 +651,11 @@ __device__ bool solve_group(const hf_scene* __restrict__ scenes, const TileItem*
                     part[0] += (double)pc * (double)ap;
                 }
                 group_sum<1>(part, red);   // its __syncthreads also ends every read of the slot
-                if (lt == 0) bufA[c] = part[0];
+                if (lt == 0) bufA[placed(nth, ti.scene, c)] = part[0];
             };
             pipelined_tiles(first, tile_hi, nlb, loc, scene_lo, tiles, slots, mbar, ph, ws.err, issue, work);
         }
-        for (int c = first; !TMA && c < tile_hi; c += nlb) {
+        for (int c = first, nth = 0; !TMA && c < tile_hi; c += nlb, ++nth) {
             const TileItem ti = tiles[c];
             const LocalScene& L = loc[ti.scene - scene_lo];
             if (!L.live) continue;
@@ -645,7 +689,7 @@ __device__ bool solve_group(const hf_scene* __restrict__ scenes, const TileItem*
                 part[0] += (double)pc[m] * (double)ap[m];
             }
             group_sum<1>(part, red);
-            if (lt == 0) bufA[c] = part[0];
+            if (lt == 0) bufA[placed(nth, ti.scene, c)] = part[0];
         }
         if (!(ok = grid_barrier(bar, epoch, ws.err, nlb))) goto done;
         {
@@ -675,7 +719,7 @@ __device__ bool solve_group(const hf_scene* __restrict__ scenes, const TileItem*
                     tma_load_3d(slot + 4096, &M[11], ti.k0, ti.j0, ti.i0, mb);
                 }
             };
-            auto work = [&](int c, float* slot) {
+            auto work = [&](int c, float* slot, int nth) {
                 const TileItem ti = tiles[c];
                 const LocalScene& L = loc[ti.scene - scene_lo];
                 const hf_scene& S = scenes[ti.scene];
@@ -698,13 +742,14 @@ __device__ bool solve_group(const hf_scene* __restrict__ scenes, const TileItem*
                 }
                 group_sum<2>(part, red);
                 if (lt == 0) {
-                    bufB[1 * ws.tiles + c] = part[0];
-                    bufB[2 * ws.tiles + c] = part[1];
+                    const int at = placed(nth, ti.scene, c);
+                    bufB[1 * ws.tiles + at] = part[0];
+                    bufB[2 * ws.tiles + at] = part[1];
                 }
             };
             pipelined_tiles(first, tile_hi, nlb, loc, scene_lo, tiles, slots, mbar, ph, ws.err, issue, work);
         }
-        for (int c = first; !TMA && c < tile_hi; c += nlb) {
+        for (int c = first, nth = 0; !TMA && c < tile_hi; c += nlb, ++nth) {
             const TileItem ti = tiles[c];
             const LocalScene& L = loc[ti.scene - scene_lo];
             if (!L.live) continue;
@@ -739,8 +784,9 @@ __device__ bool solve_group(const hf_scene* __restrict__ scenes, const TileItem*
             }
             group_sum<2>(part, red);
             if (lt == 0) {
-                bufB[1 * ws.tiles + c] = part[0];
-                bufB[2 * ws.tiles + c] = part[1];
+                const int at = placed(nth, ti.scene, c);
+                bufB[1 * ws.tiles + at] = part[0];
+                bufB[2 * ws.tiles + at] = part[1];
             }
         }
         if (!(ok = grid_barrier(bar, epoch, ws.err, nlb))) goto done;
@@ -784,7 +830,7 @@ __device__ bool solve_group(const hf_scene* __restrict__ scenes, const TileItem*
             part[0] += rt * rt;
         }
         group_sum<1>(part, red);
-        if (lt == 0) bufA[1 * ws.tiles + c] = part[0];
+        if (lt == 0) bufA[1 * ws.tiles + part_at(ws.tile_begin, ti.scene, c)] = part[0];
     }
     if (!(ok = grid_barrier(bar, epoch, ws.err, nlb))) goto done;
     for (int q = 0; q < ns; ++q) {
@@ -837,8 +883,9 @@ __device__ bool solve_group(const hf_scene* __restrict__ scenes, const TileItem*
         }
         group_sum<2>(part, red);
         if (lt == 0) {
-            bufB[1 * ws.tiles + c] = part[0];
-            bufB[2 * ws.tiles + c] = part[1];
+            const int at = part_at(ws.tile_begin, ti.scene, c);
+            bufB[1 * ws.tiles + at] = part[0];
+            bufB[2 * ws.tiles + at] = part[1];
         }
     }
     if (!(ok = grid_barrier(bar, epoch, ws.err, nlb))) goto done;
@@ -898,6 +945,7 @@ __global__ void __launch_bounds__(kThreads) k_pcg(const hf_scene* __restrict__ s
     __shared__ LocalScene loc[kGroupScenes];
     __shared__ unsigned char s_par[kGroupScenes];
     __shared__ int s_any;
+    __shared__ int place[kPlaces];
     __shared__ __align__(8) unsigned long long mbar[2];
     extern __shared__ __align__(128) float sm_raw[];
     float* slots = TMA ? align128_shared(sm_raw) : nullptr;
@@ -920,7 +968,7 @@ __global__ void __launch_bounds__(kThreads) k_pcg(const hf_scene* __restrict__ s
         const int g = *(volatile int*)next;
         if (g >= gt.count) break;
         if (!solve_group<HEAT, TMA>(scenes, tiles, gt.g[g], lb, nlb, bar, epoch, dt_d, ws, red, loc, s_par, &s_any, slots,
-                                    mbar, ph))
+                                    mbar, ph, place))
             break;
     }
     // a timed-out barrier leaves the groups that no lane reached unsolved: flag their scenes

@@ -139,3 +139,16 @@ def test_quotient_is_the_operators():
         got = out.cpu().numpy()
         bad = (got.view(np.int64) != want.view(np.int64)) & ~(np.isnan(got) & np.isnan(want))
         assert not bad.any(), (int(bad.sum()), a[bad][0].hex(), b[bad][0].hex(), got[bad][0].hex(), want[bad][0].hex())
+
+
+@pytest.mark.parametrize("sizes,blocks,lanes", [((70,), 3, 0), ((70,), 0, 0), ((97, 33, 150), 2, 1), ((50, 49, 53, 54), 8, 2)], ids=str)
+def test_streaming_sums_by_units(sizes, blocks, lanes):
+    """The streaming kernel's scene sums, whose partials are spread by unit, for blocks of more tiles than keep their places (162
+    and 2072 of them), units of one tile and of one and two, and scenes that share a lane: the on-chip solve's bits."""
+    from heatflow_mpm.scene import ScenePlan
+    chip, stream = _scenes(sizes, 75), _scenes(sizes, 75)
+    for plan in (ScenePlan(chip), ScenePlan(stream, streaming_cg=True, persistent_blocks=blocks, lanes=lanes)):
+        plan.prepare_statics()
+        plan.substep(2e-3)
+    for a, b in zip(chip, stream):
+        _equal(a, b)
