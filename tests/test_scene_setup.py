@@ -258,11 +258,3 @@ def test_mesh_particles_fill(tmp_path):
     assert np.linalg.norm(P - c, axis=1).max() < 0.03 + 2.5e-3
     again = mesh_particles(str(p), height=0.06, spacing=2.5e-3, L=0.24, seed=2)
     assert np.array_equal(P, again)
-
-
-def test_scene_carries_no_array_that_no_solve_reads():
-    """The cell-layout copy of the z face diffusivities has no reader left: a scene neither allocates it nor has it written."""
-    from heatflow_mpm.scene import DeviceScene, SceneSpec
-    sc = DeviceScene(SceneSpec(n=8, h=0.01), "cpu")
-    sc.fill_record()
-    assert not sc.record.hkzc and sc.record.hkz and sc.record.ayc and sc.record.azc
