@@ -5,7 +5,7 @@
 // solve (heat.py:198-210).  A team of blocks (one per SM) owns a scene's tiles in contiguous runs of whole units; r, A p
 // (and D) of a block's cells live in registers, p and x in shared memory, so an iteration moves only what blocks owe each
 // other.  A plan of several scenes gives every scene a team of its own and a place in the blocks' common order
-// (brick_schedule, hf_api.cu); teams work side by side.
+// (brick_teams and brick_jobs, hf_api.cu); teams work side by side.
 //
 // What bounds an iteration: two reductions of the whole scene (p.Ap; r.r and r.z), one halo exchange, and between them the
 // issue of some 90 instructions per cell (96^3: 16,300 cycles, of which 7,800 for the exchanges; 45 % issue).  A barrier

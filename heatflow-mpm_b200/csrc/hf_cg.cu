@@ -596,8 +596,7 @@ __device__ bool solve_group(const hf_scene* __restrict__ scenes, const TileItem*
     for (int kit = 1; *s_any; ++kit) {
         // phase A: p_k at the stencil points, Ap = A p_k, p.Ap
         if constexpr (TMA) {
-            // stage z and p_{k-1} with a one-cell halo and the tile's face fractions (the resident kernel's box
-            // geometry), form p_k in place, A p from shared memory
+            // stage z and p_{k-1} with a one-cell halo and the tile's face fractions, form p_k in place, A p from shared memory
             const bool first_it = kit == 1;
             auto issue = [&](int c, float* slot, unsigned long long* mb) {
                 const TileItem ti = tiles[c];

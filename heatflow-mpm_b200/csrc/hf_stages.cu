@@ -248,10 +248,10 @@ __device__ __forceinline__ void coeff_cell(const hf_scene& S, float afmin, float
         hkzv = face_kappa(conductivity(an, ka, km), kc);
     }
     S.hkz[fw] = hkzv;
-    if (S.hkzc) S.hkzc[t] = hkzv;   // cell-layout copy for the tiled (TMA) heat stencil
+    if (S.hkzc) S.hkzc[t] = hkzv;   // copy in cell layout; no solve of this library reads it
     S.ay[fv] = ayv;
     S.az[fw] = azv;
-    S.ayc[t] = ayv;   // cell-layout copies for the tiled (TMA) pressure stencil
+    S.ayc[t] = ayv;   // cell-layout copies for the streaming solve's tiled (TMA) pressure stencil
     S.azc[t] = azv;
     if (i == n - 1) S.ax[uidx(n, n, j, k)] = S.hkx[uidx(n, n, j, k)] = 0.0f;
     if (j == n - 1) S.ay[vidx(n, i, n, k)] = S.hky[vidx(n, i, n, k)] = 0.0f;
